@@ -771,7 +771,18 @@ int compile_bend(const trk_lattice *l, int idx, double Po, trk_op *op, std::vect
   for (int j = 0; j < nSub; j++) {
     d[BD_OMC + j] = 2 * d[BD_SH + j] * d[BD_SH + j];
     d[BD_C1 + j] = d[BD_DS + j] * d[BD_INVRHOA];
-    d[BD_C2 + j] = d[BD_C1 + j] * d[BD_RHOINV];
+    /* rounded once: the merged body's whole kick is C2 (rho0 + X) */
+    d[BD_C2 + j] = (double)((long double)d[BD_DS + j] / ((long double)rho_actual * rho0));
+  }
+  if (nSub == 4) {
+    const long double rho = rho0, a0 = d[BD_DSH] / rho, a1 = d[BD_DSH + 1] / rho;
+    d[BD_SA2] = (double)sinl(2 * a0);
+    d[BD_CA2] = (double)cosl(2 * a0);
+    d[BD_OMC2] = (double)(2 * sinl(a0) * sinl(a0));
+    /* a slice turns by 2 a0 + 2 a1: the inner drifts, whose sine has the
+     * smaller ulp, take up the rounding of the outer's */
+    d[BD_SA1] = (double)sinl(a1 + (2 * a0 - asinl((long double)d[BD_SA2])) / 2);
+    d[BD_KT] = (double)((2 * (long double)d[BD_DS] + d[BD_DS + 1]) / (rho * rho_actual));
   }
   return TRK_OK;
 }
@@ -1034,7 +1045,17 @@ int trk_compile(const trk_lattice *l, double Po, CompiledLattice &out) {
       else if (plain && op.i[2] == 1 && op.i[3] == 5) {
         op.kind = OPK_CFBEND;
         out.has_cfbend = true;
+        const double *Fy = out.field.data() + op.i[4] + 121;
+        if (Fy[2 * 11] == 0 && Fy[3 * 11] == 0 && Fy[4 * 11] == 0)
+          op.i[7] |= BF_LINEAR;
       }
+      /* the merged bodies take |q| up to 2^-6: inside a slice the design
+       * orbit swings to 0.8512 of the slice angle (the fourth-order
+       * integrator's overshoot after the second kick); below 0.010 a particle
+       * keeps more than 5e-3 for its own slope.  Bends of larger slice angles
+       * go to the checked bodies at once rather than through both. */
+      if (plain && 0.8512 * std::fabs(op.d[BD_SLICE] / op.d[BD_RHO0]) < 0.010)
+        op.i[7] |= BF_MERGED;
     }
     if (op.kind != OPK_NOP && op.kind != OPK_DRIFT && op.kind != OPK_EDRIFT && op.kind != OPK_RFDRIFT &&
         op.kind != OPK_MULT1 && op.kind != OPK_DIPOLE && op.kind != OPK_CFBEND && op.kind != OPK_RF &&

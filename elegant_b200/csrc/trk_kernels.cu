@@ -66,6 +66,16 @@ struct Part {
 
 __device__ __forceinline__ double sqr(double v) { return v * v; }
 
+/* a particle and whether it was lost, as the out-of-line paths return it */
+struct PartLoss {
+  Part p;
+  int lost;
+};
+
+/* high word of |v|: orders like |v|, infinities and NaN above every number */
+__device__ __forceinline__ unsigned hi_abs(double v) { return (unsigned)__double2hiint(v) & 0x7fffffffu; }
+__device__ __forceinline__ bool finite2(double u, double v) { return max(hi_abs(u), hi_abs(v)) < 0x7ff00000u; }
+
 #if TRK_FAST
 /* Reciprocal and square root for the fast build: the hardware approximation
  * y0 (about 20 correct bits) and one third-order correction from the series
@@ -2191,6 +2201,379 @@ __device__ __forceinline__ void op_dipole_fast2(const trk_op *__restrict__ op, P
 }
 #endif
 
+#if TRK_FAST
+/* ------------------------------------------ merged fast-build bodies
+ * The fast build's bodies of OPK_MULT1, OPK_DIPOLE and OPK_CFBEND for the
+ * particles that matter: momenta small against the total momentum, positions
+ * clear of every loss limit.  Two identities of exact arithmetic take
+ * operations out of the integrator:
+ *  - a slice ends with the drift the next slice begins with, and two drifts
+ *    in a row are one (a straight line; in a bend, rotation angles add), so a
+ *    slice costs three drifts and three kicks instead of four and three;
+ *  - in momenta divided by the constant total momentum the square roots are
+ *    functions of z = px^2 + py^2 alone,
+ *      (1 - z)^(-1/2) = 1 + sec_m1(z),  (1 - z)^(1/2) = 1 - cos_m1(z),
+ *    and for z <= 2^-12 three terms reach FP64 accuracy: no reciprocal or
+ *    root per substep, and a chain of multiply-adds instead of two dependent
+ *    hardware approximations.
+ * The loss conditions of the element (undefined slopes, |QX| > f, limits on
+ * coordinates and slopes, the per-slice aperture) are excluded by bounds kept
+ * on the way as integer maxima of high words (ALU pipe): a particle that
+ * comes near any of them leaves the body unchanged and takes the checked one
+ * (op_mult1_fast and so on), which locates the loss as the reference does.
+ * Bound by FP64 issue and by the length of the substep's chain (13 of its 17
+ * operations).  Measured against the checked bodies alone, ms per turn: FODO
+ * ring with RF and wake, 1e6 particles, 11.4 -> 7.6; achromat ring, 2e6, 250
+ * -> 169; FODO ring, 1e4 particles, 0.67 -> 0.41; dynamic-aperture grids over
+ * 24 seeds, where the checked bodies divide for the aperture in every slice,
+ * 101 -> 46 for 32 turns. */
+
+/* Coefficients: the power series, its first omitted term economized over
+ * [0, b], b = 2^-12 (z^4 replaced by z^4 - b^4 T4*(z/b)/128 without the
+ * constant b^4/128): error below 2e-17 of 1. */
+#define TRK_Z_B 0x1p-12
+#define TRK_Z_HI 0x3f300000u /* high word of 2^-12 */
+#define TRK_ECON3(a3, a4) ((a3) + 2 * TRK_Z_B * (a4))
+#define TRK_ECON2(a2, a4) ((a2) - 1.25 * TRK_Z_B * TRK_Z_B * (a4))
+#define TRK_ECON1(a1, a4) ((a1) + 0.25 * TRK_Z_B * TRK_Z_B * TRK_Z_B * (a4))
+__device__ __forceinline__ double sec_m1(double z) {
+  const double a4 = 35.0 / 128;
+  return z * fma(z, fma(z, TRK_ECON3(5.0 / 16, a4), TRK_ECON2(3.0 / 8, a4)), TRK_ECON1(1.0 / 2, a4));
+}
+__device__ __forceinline__ double cos_m1(double z) {
+  const double a4 = 5.0 / 128;
+  return z * fma(z, fma(z, TRK_ECON3(1.0 / 16, a4), TRK_ECON2(1.0 / 8, a4)), TRK_ECON1(1.0 / 2, a4));
+}
+
+/* a double above every |v| whose high word is h */
+__device__ __forceinline__ double above(unsigned h) { return __hiloint2double((int)(h + 1), 0); }
+
+/* limits on |x|, |y| at the element's ends and 1 + delta > 0, by high word:
+ * below 8 (the reference's limit is 10) and in (2^-31, 2^1000) */
+#define TRK_COORD_HI 0x40200000u
+__device__ __forceinline__ bool momentum_plain(double opd) {
+  const int h = __double2hiint(opd);
+  return h > 0x3e000000 && h < 0x7e700000;
+}
+
+/* true if every point of the box |x| <= xb, |y| <= yb passes check_aperture:
+ * its elliptical test in products, with a margin above their roundings */
+__device__ __forceinline__ bool box_inside(double xb, double yb, const trk_aperture *__restrict__ ap) {
+  const double xmax = __ldg(&ap->x_max), ymax = __ldg(&ap->y_max);
+  if (__ldg(&ap->elliptical) && xmax > 0 && ymax > 0) {
+    if (__ldg(&ap->xexp) != 2 || __ldg(&ap->yexp) != 2)
+      return false;
+    const double a2 = xmax * xmax, b2 = ymax * ymax;
+    return fma(xb * xb, b2, yb * yb * a2) < a2 * b2 * (1 - 0x1p-40);
+  }
+  return (!(xmax > 0) || xb < xmax) && (!(ymax > 0) || yb < ymax);
+}
+
+/* k / opd to half an ulp.  A relative error of the bend's kick moves the
+ * closed orbit by the dispersion times it, 1e-12 of a beam size for an ulp,
+ * so the bends round a slice's whole kick once and take the second kick,
+ * 1.7 times as large and opposite, as what the two others leave of it. */
+__device__ __forceinline__ double kick_over(double k, double opd, double iopd) {
+  const double q = k * iopd;
+  return fma(fma(-q, opd, k), iopd, q);
+}
+
+/* OPK_MULT1; false: not taken, p unchanged.  Per kick: 2 to 8 operations of
+ * the kick, 9 of the drift (13 and 15 in the unmerged body, with a reciprocal
+ * square root). */
+template <int ORDER>
+__device__ __forceinline__ bool mult1_merged(const double *__restrict__ d, int n_parts, Part &p,
+                                             const trk_aperture *__restrict__ ap) {
+  const double opd = 1 + p.dp, iopd = rcp_fast(opd);
+  const double ss = fma(p.yp, p.yp, fma(p.xp, p.xp, 1.0));
+  const double r0 = rsqrt_fast(ss);
+  double x = p.x, y = p.y, px = p.xp * r0, py = p.yp * r0;
+  const double l0 = __ldg(&d[MD_DSH]), l1 = __ldg(&d[MD_DSH + 1]);
+  const double ka = kick_over(__ldg(&d[MD_KQ]), opd, iopd), kb = kick_over(__ldg(&d[MD_KQ + 3]), opd, iopd);
+  unsigned zm = 0, xm = hi_abs(x), ym = hi_abs(y);
+  double s = l0 * (ss * r0), v = 0; /* first drift: slopes xp, sqrt(1 + xp^2 + yp^2) */
+  x = fma(p.xp, l0, x);
+  y = fma(p.yp, l0, y);
+#define TRK_KICK(K)                                                                                          \
+  {                                                                                                          \
+    xm = max(xm, hi_abs(x));                                                                                 \
+    ym = max(ym, hi_abs(y));                                                                                 \
+    if (ORDER == 1) {                                                                                        \
+      px = fma(-(K), x, px);                                                                                 \
+      py = fma((K), y, py);                                                                                  \
+    } else if (ORDER == 2) {                                                                                 \
+      px = fma(-0.5 * (K), fma(x, x, -y * y), px);                                                           \
+      py = fma((K), x * y, py);                                                                              \
+    } else {                                                                                                 \
+      const double x2 = x * x, y2 = y * y, k6 = (K) * (1.0 / 6);                                             \
+      px = fma(-k6, fma(-3.0, y2, x2) * x, px);                                                              \
+      py = fma(k6, fma(3.0, x2, -y2) * y, py);                                                               \
+    }                                                                                                        \
+  }
+#define TRK_DRIFT(L)                                                                                         \
+  {                                                                                                          \
+    const double z = fma(py, py, px * px);                                                                   \
+    zm = max(zm, (unsigned)__double2hiint(z));                                                               \
+    v = sec_m1(z);                                                                                           \
+    const double l = fma((L), v, (L));                                                                       \
+    x = fma(px, l, x);                                                                                       \
+    y = fma(py, l, y);                                                                                       \
+    s += l;                                                                                                  \
+  }
+  for (int i = 1; i <= n_parts; i++) {
+    const double le = i < n_parts ? 2 * l0 : l0;
+    TRK_KICK(ka)
+    TRK_DRIFT(l1)
+    TRK_KICK(kb)
+    TRK_DRIFT(l1)
+    TRK_KICK(ka)
+    TRK_DRIFT(le)
+  }
+#undef TRK_KICK
+#undef TRK_DRIFT
+  xm = max(xm, hi_abs(x));
+  ym = max(ym, hi_abs(y));
+  if (!(zm < TRK_Z_HI && max(xm, ym) < TRK_COORD_HI && momentum_plain(opd)))
+    return false;
+  /* every slice boundary lies on a straight segment between these points */
+  if (ap && !box_inside(above(xm), above(ym), ap))
+    return false;
+  p.x = x;
+  p.y = y;
+  p.xp = fma(px, v, px);
+  p.yp = fma(py, v, py);
+  p.s += s;
+  return true;
+}
+
+/* OPK_DIPOLE, momenta in units of 1 + delta: px and the constant py, pz =
+ * sqrt(1 - px^2 - py^2).  The drift through the angle a as in dipole_slice,
+ * with pz = 1 - cos_m1(z) before it and 1/pz = 1 + sec_m1(z) after it; Y and
+ * the path grow by py and 1 times the sum F of the drifts' lengths; the kick
+ * is px -= k R with R = rho0 + X, k = ds/(rho_actual rho0 (1 + delta)).  17
+ * operations per kick and drift (20 with a root and a reciprocal in the
+ * unmerged body). */
+__device__ __forceinline__ bool dipole_merged(const double *__restrict__ d, int nSlices, Part &p,
+                                              const trk_aperture *__restrict__ ap) {
+  const double rho0 = __ldg(&d[BD_RHO0]);
+  const double opd = 1 + p.dp, iopd = rcp_fast(opd);
+  const double r0 = rsqrt_fast(fma(p.yp, p.yp, fma(p.xp, p.xp, 1.0)));
+  const double py = p.yp * r0, py2 = py * py;
+  double px = p.xp * r0, X = p.x, F = 0, v = 0;
+  const double ka = kick_over(__ldg(&d[BD_C2]), opd, iopd);
+  const double kb = fma(-2.0, ka, kick_over(__ldg(&d[BD_KT]), opd, iopd));
+  const double s1 = __ldg(&d[BD_SA1]), c1 = __ldg(&d[BD_CA + 1]), m1 = __ldg(&d[BD_OMC + 1]);
+  const double s2 = __ldg(&d[BD_SA2]), c2 = __ldg(&d[BD_CA2]), m2 = __ldg(&d[BD_OMC2]);
+  unsigned zm = 0, xm = hi_abs(X);
+  double R = rho0 + X;
+#define TRK_DRIFT(SA, CA, OMC)                                                                               \
+  {                                                                                                          \
+    const double z = fma(px, px, py2), h = cos_m1(z);                                                        \
+    const double m = fma(-(OMC), h, fma((SA), px, (OMC)));                                                   \
+    px = fma(-(SA), h, fma((CA), px, (SA)));                                                                 \
+    const double z1 = fma(px, px, py2);                                                                      \
+    v = sec_m1(z1);                                                                                          \
+    zm = max(zm, max((unsigned)__double2hiint(z), (unsigned)__double2hiint(z1)));                            \
+    const double u = fma(R, v, R);                                                                           \
+    X = fma(u, m, X);                                                                                        \
+    F = fma(u, (SA), F);                                                                                     \
+    R = rho0 + X;                                                                                            \
+    xm = max(xm, hi_abs(X));                                                                                 \
+  }
+  {
+    const double s0 = __ldg(&d[BD_SA]), c0 = __ldg(&d[BD_CA]), m0 = __ldg(&d[BD_OMC]);
+    TRK_DRIFT(s0, c0, m0)
+  }
+  for (int i = 1; i <= nSlices; i++) {
+    px = fma(-ka, R, px);
+    TRK_DRIFT(s1, c1, m1)
+    px = fma(-kb, R, px);
+    TRK_DRIFT(s1, c1, m1)
+    px = fma(-ka, R, px);
+    if (i < nSlices)
+      TRK_DRIFT(s2, c2, m2)
+  }
+  {
+    const double s0 = __ldg(&d[BD_SA]), c0 = __ldg(&d[BD_CA]), m0 = __ldg(&d[BD_OMC]);
+    TRK_DRIFT(s0, c0, m0)
+  }
+#undef TRK_DRIFT
+  const double Y = fma(py, F, p.y);
+  if (!(zm < TRK_Z_HI && max(xm, max(hi_abs(p.y), hi_abs(Y))) < TRK_COORD_HI && momentum_plain(opd)))
+    return false;
+  if (ap) {
+    /* a slice boundary lies on a chord between two of these points, at most
+     * R (1 - cos a) nearer the centre; with |X| below rho0/8 the path grows
+     * from slice to slice, so Y stays between its ends */
+    const double xb = above(xm);
+    if (!(xb < 0.125 * fabs(rho0)) ||
+        !box_inside(fma(2 * fabs(rho0), m2, xb), above(max(hi_abs(p.y), hi_abs(Y))), ap))
+      return false;
+  }
+  p.x = X;
+  p.y = Y;
+  p.xp = fma(px, v, px);
+  p.yp = fma(py, v, py);
+  p.s += F;
+  return true;
+}
+
+/* OPK_CFBEND: the same with kicks that change py.  The field as in cf_fields;
+ * LIN: K1 only, the midplane field linear in x. */
+template <bool LIN>
+__device__ __forceinline__ bool cfbend_merged(const double *__restrict__ d, const double *__restrict__ fxy, int nSlices,
+                                              Part &p, const trk_aperture *__restrict__ ap) {
+  const double rho0 = __ldg(&d[BD_RHO0]);
+  const double opd = 1 + p.dp, iopd = rcp_fast(opd);
+  const double r0 = rsqrt_fast(fma(p.yp, p.yp, fma(p.xp, p.xp, 1.0)));
+  double px = p.xp * r0, py = p.yp * r0, X = p.x, Y = p.y, dist = 0, v = 0;
+  const double ca = kick_over(__ldg(&d[BD_C2]), opd, iopd);
+  const double cb = fma(-2.0, ca, kick_over(__ldg(&d[BD_KT]), opd, iopd));
+  unsigned zm = 0, xm = hi_abs(X), ym = hi_abs(Y);
+  double R = rho0 + X, py2 = py * py;
+#define CF_T(T, i, j) __ldg(&(T)[(i) * 11 + (j)])
+#define TRK_DRIFT(S, C, O)                                                                                   \
+  {                                                                                                          \
+    const double sa = __ldg(&dd[S]), co = __ldg(&dd[C]), omc = __ldg(&dd[O]);                                \
+    const double z = fma(px, px, py2), h = cos_m1(z);                                                        \
+    const double m = fma(-omc, h, fma(sa, px, omc));                                                         \
+    px = fma(-sa, h, fma(co, px, sa));                                                                       \
+    const double z1 = fma(px, px, py2);                                                                      \
+    v = sec_m1(z1);                                                                                          \
+    zm = max(zm, max((unsigned)__double2hiint(z), (unsigned)__double2hiint(z1)));                            \
+    const double u = fma(R, v, R), us = u * sa;                                                              \
+    X = fma(u, m, X);                                                                                        \
+    Y = fma(py, us, Y);                                                                                      \
+    dist += us;                                                                                              \
+    R = rho0 + X;                                                                                            \
+    xm = max(xm, hi_abs(X));                                                                                 \
+    ym = max(ym, hi_abs(Y));                                                                                 \
+  }
+#define TRK_KICK(K)                                                                                          \
+  {                                                                                                          \
+    const double y2 = Y * Y;                                                                                 \
+    const double *Tx = ff, *Ty = ff + 121;                                                                   \
+    const double p0 =                                                                                        \
+      LIN ? fma(CF_T(Ty, 1, 0), X, CF_T(Ty, 0, 0))                                                           \
+          : fma(fma(fma(fma(CF_T(Ty, 4, 0), X, CF_T(Ty, 3, 0)), X, CF_T(Ty, 2, 0)), X, CF_T(Ty, 1, 0)), X,   \
+                CF_T(Ty, 0, 0));                                                                             \
+    const double p2 = fma(fma(CF_T(Ty, 2, 2), X, CF_T(Ty, 1, 2)), X, CF_T(Ty, 0, 2));                        \
+    const double fy = fma(y2, fma(y2, CF_T(Ty, 0, 4), p2), p0);                                              \
+    const double q1 = fma(fma(fma(CF_T(Tx, 3, 1), X, CF_T(Tx, 2, 1)), X, CF_T(Tx, 1, 1)), X, CF_T(Tx, 0, 1)); \
+    const double q3 = fma(CF_T(Tx, 1, 3), X, CF_T(Tx, 0, 3));                                                \
+    const double wk = (K) * R;                                                                               \
+    px = fma(-wk, fy, px);                                                                                   \
+    py = fma(wk * Y, fma(y2, q3, q1), py);                                                                   \
+    py2 = py * py;                                                                                           \
+  }
+  {
+    const double *dd = d;
+    TRK_DRIFT(BD_SA, BD_CA, BD_OMC)
+  }
+  for (int i = 1; i <= nSlices; i++) {
+    /* the tables are read again every slice (L1) rather than held in registers */
+    const double *dd = d, *ff = fxy;
+    asm volatile("" : "+l"(dd), "+l"(ff));
+    TRK_KICK(ca)
+    TRK_DRIFT(BD_SA1, BD_CA + 1, BD_OMC + 1)
+    TRK_KICK(cb)
+    TRK_DRIFT(BD_SA1, BD_CA + 1, BD_OMC + 1)
+    TRK_KICK(ca)
+    if (i < nSlices)
+      TRK_DRIFT(BD_SA2, BD_CA2, BD_OMC2)
+  }
+  {
+    const double *dd = d;
+    TRK_DRIFT(BD_SA, BD_CA, BD_OMC)
+  }
+#undef TRK_KICK
+#undef TRK_DRIFT
+#undef CF_T
+  if (!(zm < TRK_Z_HI && max(xm, ym) < TRK_COORD_HI && momentum_plain(opd)))
+    return false;
+  if (ap) {
+    /* as in dipole_merged; Y runs along the same chords */
+    const double xb = above(xm);
+    if (!(xb < 0.125 * fabs(rho0)) ||
+        !box_inside(fma(2 * fabs(rho0), __ldg(&d[BD_OMC2]), xb), above(ym), ap))
+      return false;
+  }
+  p.x = X;
+  p.y = Y;
+  p.xp = fma(px, v, px);
+  p.yp = fma(py, v, py);
+  p.s += dist;
+  return true;
+}
+
+/* The checked bodies out of line for the particles the merged ones leave,
+ * passed and returned by value (a reference would pin the caller's
+ * coordinates in local memory). */
+__device__ __noinline__ PartLoss mult1_checked(const trk_op *__restrict__ op, Part p, double Po, double z_start,
+                                               const trk_aperture *ap) {
+  PartLoss r;
+  r.lost = !op_mult1_fast(op, p, Po, z_start, ap);
+  r.p = p;
+  return r;
+}
+
+__device__ __noinline__ PartLoss dipole_checked(const trk_op *__restrict__ op, Part p, double Po, double z_start,
+                                                const trk_aperture *ap) {
+  PartLoss r;
+  r.lost = !op_dipole_fast(op, p, Po, z_start, ap);
+  r.p = p;
+  return r;
+}
+
+__device__ __noinline__ PartLoss cfbend_checked(const trk_op *__restrict__ op, Part p, double Po, double z_start,
+                                                const trk_aperture *ap, const double *__restrict__ field) {
+  PartLoss r;
+  r.lost = !op_cfbend_fast(op, p, Po, z_start, ap, field);
+  r.p = p;
+  return r;
+}
+
+__device__ __forceinline__ bool op_mult1(const trk_op *__restrict__ op, Part &p, double Po, double z_start,
+                                         const trk_aperture *ap) {
+  const int n_parts = __ldg(&op->i[0]), order = __ldg(&op->i[4]) & 0xff;
+  bool done;
+  if (order == 1)
+    done = mult1_merged<1>(op->d, n_parts, p, ap);
+  else if (order == 2)
+    done = mult1_merged<2>(op->d, n_parts, p, ap);
+  else
+    done = mult1_merged<3>(op->d, n_parts, p, ap);
+  if (done)
+    return true;
+  const PartLoss r = mult1_checked(op, p, Po, z_start, ap);
+  p = r.p;
+  return !r.lost;
+}
+
+__device__ __forceinline__ bool op_dipole(const trk_op *__restrict__ op, Part &p, double Po, double z_start,
+                                          const trk_aperture *ap) {
+  if ((__ldg(&op->i[7]) & BF_MERGED) && dipole_merged(op->d, __ldg(&op->i[0]), p, ap))
+    return true;
+  const PartLoss r = dipole_checked(op, p, Po, z_start, ap);
+  p = r.p;
+  return !r.lost;
+}
+
+__device__ __forceinline__ bool op_cfbend(const trk_op *__restrict__ op, Part &p, double Po, double z_start,
+                                          const trk_aperture *ap, const double *__restrict__ field) {
+  const int flags = __ldg(&op->i[7]);
+  if (flags & BF_MERGED) {
+    const double *fxy = field + __ldg(&op->i[4]);
+    if ((flags & BF_LINEAR) ? cfbend_merged<true>(op->d, fxy, __ldg(&op->i[0]), p, ap)
+                            : cfbend_merged<false>(op->d, fxy, __ldg(&op->i[0]), p, ap))
+      return true;
+  }
+  const PartLoss r = cfbend_checked(op, p, Po, z_start, ap, field);
+  p = r.p;
+  return !r.lost;
+}
+#endif
+
 /* ------------------------------------------------------ after-element */
 /* limit_amplitudes / elimit_amplitudes (src/limit_amplitudes.c:197-288,
  * 487-~620) for one particle; returns true if lost. */
@@ -2264,17 +2647,18 @@ __device__ __forceinline__ bool post_aperture_body(Part &p, const trk_aperture *
  * reference's arithmetic); anything else goes to post_aperture_full. */
 __device__ __forceinline__ bool post_aperture_inside(const Part &p, const trk_aperture *__restrict__ ap) {
   const double xmax = __ldg(&ap->x_max), ymax = __ldg(&ap->y_max);
-  if (!(isfinite(p.x) && isfinite(p.y)))
+  if (!finite2(p.x, p.y))
     return false;
-  if (__ldg(&ap->elliptical) && xmax > 0 && ymax > 0)
-    return (ipow_d(p.x, __ldg(&ap->xexp)) / __ldg(&ap->a2) + ipow_d(p.y, __ldg(&ap->yexp)) / __ldg(&ap->b2)) <= 1;
+  if (__ldg(&ap->elliptical) && xmax > 0 && ymax > 0) {
+    /* x^2/a2 + y^2/b2 <= 1 in products, with a margin above the roundings of
+     * either form (an overflowing a2 b2 still exceeds a finite left side) */
+    if (__ldg(&ap->xexp) != 2 || __ldg(&ap->yexp) != 2)
+      return (ipow_d(p.x, __ldg(&ap->xexp)) / __ldg(&ap->a2) + ipow_d(p.y, __ldg(&ap->yexp)) / __ldg(&ap->b2)) <= 1;
+    const double a2 = __ldg(&ap->a2), b2 = __ldg(&ap->b2);
+    return fma(p.x * p.x, b2, (p.y * p.y) * a2) < (a2 * b2) * (1 - 0x1p-40);
+  }
   return (!(xmax > 0) || fabs(p.x) <= xmax) && (!(ymax > 0) || fabs(p.y) <= ymax);
 }
-
-struct PartLoss {
-  Part p;
-  int lost;
-};
 
 /* Out of line, with the particle passed and returned by value (a reference
  * would pin the caller's coordinates in local memory): it only runs for
@@ -2387,7 +2771,7 @@ __device__ __forceinline__ bool after_element(const TrackArgs &a, const OpHead &
                                               long pass) {
   if (ok && !h.no_aperture && h.ap_post >= 0 && !a.element_only)
     ok = !post_aperture(p, a.aps + h.ap_post, h.extrapolate, h.z_end, a.Po);
-  if (ok && !a.element_only && (isinf(p.x) || isinf(p.y) || isnan(p.x) || isnan(p.y))) {
+  if (ok && !a.element_only && !finite2(p.x, p.y)) {
     p.s = h.z_end;
     p.dp = a.Po * (1 + p.dp);
     ok = false;
@@ -2422,14 +2806,14 @@ __device__ __forceinline__ bool track_particle(const TrackArgs &a, const trk_op 
         break;
       case OPK_MULT1:
 #if TRK_FAST
-        ok = op_mult1_fast(op, p, a.Po, h.z_start, ap_in);
+        ok = op_mult1(op, p, a.Po, h.z_start, ap_in);
 #else
         ok = op_mult(op, p, a.Po, h.z_start, ap_in);
 #endif
         break;
       case OPK_DIPOLE:
 #if TRK_FAST
-        ok = op_dipole_fast(op, p, a.Po, h.z_start, ap_in);
+        ok = op_dipole(op, p, a.Po, h.z_start, ap_in);
 #else
         ok = op_dipole_exact(op, p, a.Po, h.z_start, ap_in);
 #endif
@@ -2437,7 +2821,7 @@ __device__ __forceinline__ bool track_particle(const TrackArgs &a, const trk_op 
       case OPK_CFBEND:
 #if TRK_FAST
         if (LEAN != 1)
-          ok = op_cfbend_fast(op, p, a.Po, h.z_start, ap_in, a.field);
+          ok = op_cfbend(op, p, a.Po, h.z_start, ap_in, a.field);
 #else
         if (LEAN != 1) /* flavour 1 lattices hold no combined-function bend */
           ok = op_bend(op, p, a.Po, h.z_start, ap_in, a.field);

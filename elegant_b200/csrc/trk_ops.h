@@ -61,6 +61,8 @@ enum trk_op_kind {
 #define BF_EXPAND 64   /* EXPAND_HAMILTONIAN: leading-order drift, (1+delta) coordinate factors */
 #define BF_RADE1 128   /* SYNCH_RAD with an entrance edge angle: delta pre-adjusted at the entrance */
 #define BF_RADE2 256   /* ... and post-adjusted at the exit */
+#define BF_MERGED 512  /* substep angles small enough for the fast build's merged body */
+#define BF_LINEAR 1024 /* combined function: midplane field linear in x (no K2 or higher terms) */
 
 /* RF flags (i[3]) */
 #define RF_SAME_DGAMMA 1
@@ -185,6 +187,14 @@ typedef struct {
  * the field pool after the bend's field table (at i[4], + 242 where i[2] != 0) */
 #define BD_K1F 122
 #define FR_CURV_LEN 9
+/* the last drift of a slice and the first of the next in one (fast build):
+ * sin, cos and 1 - cos of twice the first substep's angle, and the sine of the
+ * second substep's with its rounding error taken up */
+#define BD_SA2 123
+#define BD_CA2 124
+#define BD_OMC2 125
+#define BD_SA1 127
+#define BD_KT 126 /* the slice's whole kick over (rho0 + X): 2 C2[0] + C2[1] rounded once */
 /* i: 0 nSlices, 1 nSub, 2 field mode (0 dipole, 1 normal, 2 skew), 3 expansionOrder1,
  *    4 field pool offset, 5 edge1 mode, 6 edge2 mode, 7 flags */
 #define EDGE_NONE 0

@@ -1,0 +1,83 @@
+"""The fast build's merged element bodies at the edges of their range: slopes
+on both sides of 2^-6 (z = 2^-12), positions on both sides of the limits and
+of the aperture, momenta down to delta = -1, one and several slices, bends on
+both sides of the slice angle that picks the body, against the oracle."""
+import itertools
+
+import numpy as np
+import pytest
+
+from elegant_b200 import Lattice, configs
+from oracle import pyoracle
+from tests.helpers import compare, gpu_run, oracle_run
+
+pytestmark = pytest.mark.gpu
+PC = configs.P_CENTRAL
+
+# 0.8512 of the slice angle is compared with 0.010: 8 slices of 0.0117 and of 0.0118
+ELEMENTS = {
+    "quad": ("KQUAD", dict(L=0.3, K1=1.2, N_SLICES=3)),
+    "quad_one_slice": ("KQUAD", dict(L=0.3, K1=-2.0, N_SLICES=1)),
+    "sext": ("KSEXT", dict(L=0.2, K2=40.0, N_SLICES=2)),
+    "oct": ("KOCT", dict(L=0.1, K3=300.0, N_SLICES=2)),
+    "dipole": ("CSBEND", dict(L=1.0, ANGLE=0.0936, N_SLICES=8)),
+    "dipole_unmerged": ("CSBEND", dict(L=1.0, ANGLE=0.0944, N_SLICES=8)),
+    "dipole_one_slice": ("CSBEND", dict(L=0.1, ANGLE=0.008, N_SLICES=1)),
+    "bend_k1": ("CSBEND", dict(L=0.8, ANGLE=0.022, K1=-0.4, N_SLICES=4)),
+    "bend_k1k2": ("CSBEND", dict(L=0.8, ANGLE=0.03, K1=0.3, K2=5.0, N_SLICES=5)),
+}
+APERTURES = {
+    "none": None,
+    "rectangle": dict(X_MAX=0.004, Y_MAX=0.003),
+    "ellipse": dict(X_MAX=0.005, Y_MAX=0.004, ELLIPTICAL=1),
+    "superellipse": dict(X_MAX=0.005, Y_MAX=0.004, ELLIPTICAL=1, EXPONENT=4),
+}
+
+
+def _beam(aperture):
+    slopes = [0.0, 1e-5, -3e-3, 0.0156, -0.01563, 0.02]
+    if aperture == "none":
+        xs, ys, slopes = [0.0, 1e-3, -0.3, 7.99, -8.01, 9.99, 10.01], [0.0, -2e-3, 8.01], slopes + [-0.4, 0.999, 1.001]
+    else:
+        xs = [0.0, 1e-3, -0.0035, 0.00399, 0.004, -0.00401, 0.0049, 0.00501]
+        ys = [0.0, 0.0025, -0.00299, 0.00301, -0.0039]
+    rows = [(x, xp, y, yp, 0.01, d) for x, xp, y, yp, d in
+            itertools.product(xs, slopes, ys, (0.0, -2e-5, 0.0155), (0.0, 3e-3, -0.4, -0.999))]
+    rng = np.random.Generator(np.random.Philox(3))
+    jitter = rng.normal(0.0, 1e-6, (len(rows), 6)) * [1, 1, 1, 1, 1, 0]
+    rows = np.hstack([np.array(rows) + jitter, np.arange(1.0, len(rows) + 1)[:, None]])
+    return rows
+
+
+@pytest.mark.parametrize("aperture", sorted(APERTURES))
+@pytest.mark.parametrize("name", sorted(ELEMENTS))
+def test_limits_of_the_merged_bodies(tracker, name, aperture):
+    kind, params = ELEMENTS[name]
+    lat = Lattice()
+    if APERTURES[aperture]:
+        lat.add("MAXAMP", "AP", **APERTURES[aperture])
+    lat.add(kind, name, **params)
+    beam = _beam(aperture)
+    nl, g, lp, le, _ = gpu_run(tracker, lat, beam, 1, PC, fast=True)
+    with pyoracle.modes(exact_sums=True, cr_math=True):
+        rows, nlo, _ = oracle_run(lat, beam, 1, PC)
+    r = compare(g, rows, nl, nlo)
+    assert 0 < nlo and r["same_survivors"], r
+    o, gi = rows[np.argsort(rows[:, 6])], np.argsort(g[:, 6])
+    lost = o[:, 7] >= 0
+    assert np.array_equal(lp[gi][lost], o[lost, 7].astype(np.int64))
+    assert np.array_equal(le[gi][lost], o[lost, 8].astype(np.int32))
+    # each of the element's substeps rounds a few times, 2^-53 of a value of the
+    # particle's own or, in the oracle's bend drift (rho0 (cos/cos - 1)), of rho0;
+    # the steps after it carry the error on with a gain of at most a few
+    steps = 4 * params["N_SLICES"]
+    rho = params["L"] / params["ANGLE"] if kind == "CSBEND" else 1.0
+    alive = ~lost
+    ref, got = o[alive, :6], g[gi][alive, :6]
+    # a steep slope's tangent amplifies the rounding of its momentum by 1 + slope^2
+    gain = 1 + np.max(np.abs(ref[:, [1, 3]]), axis=1) ** 2
+    floor = np.array([rho, 1.0, rho, 1.0, rho, 1e-300])
+    bound = 20 * steps * 2.0 ** -53 * np.maximum(np.abs(ref), floor) * gain[:, None] ** 2
+    bound[:, 5] = 0.0  # delta passes through
+    bad = np.abs(got - ref) > bound
+    assert not bad.any(), (bad.sum(axis=0), ref[bad.any(axis=1)][:3], (got - ref)[bad.any(axis=1)][:3])
