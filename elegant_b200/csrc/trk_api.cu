@@ -93,15 +93,14 @@ struct trk_context {
   };
   std::vector<Tuned> ens_tuned;  /* autotuner choices */
   int ens_last_variant = -1;
-  /* gradient runs: pass checkpoints, element entry states, adjoints */
-  double *d_adj_ck = nullptr, *d_adj_entry = nullptr, *d_adj_lam = nullptr, *d_adj_grad = nullptr;
+  /* gradient runs: pass checkpoints, gradient, kick and field derivatives */
+  double *d_adj_ck = nullptr, *d_adj_grad = nullptr;
   double *d_adj_dk = nullptr, *d_adj_mom = nullptr;
   int *d_adj_param = nullptr;
   int *d_adj_dfo = nullptr;        /* per op: offset of a CSBEND's field derivative tables */
   double *d_adj_dfield = nullptr;  /* the tables */
   size_t adj_dfo_cap = 0, adj_dfield_cap = 0;
-  size_t adj_ck_cap = 0, adj_entry_cap = 0, adj_lam_cap = 0, adj_grad_cap = 0, adj_dk_cap = 0, adj_mom_cap = 0,
-         adj_param_cap = 0;
+  size_t adj_ck_cap = 0, adj_grad_cap = 0, adj_dk_cap = 0, adj_mom_cap = 0, adj_param_cap = 0;
   size_t matrix_cap = 0;
   double *d_gather = nullptr; /* 6 doubles per rank */
   long long *d_effort = nullptr;
@@ -841,8 +840,6 @@ void trk_context_destroy(trk_context *ctx) {
   cudaFree(ctx->d_ens_offsets);
   cudaFree(ctx->d_tune);
   cudaFree(ctx->d_adj_ck);
-  cudaFree(ctx->d_adj_entry);
-  cudaFree(ctx->d_adj_lam);
   cudaFree(ctx->d_adj_grad);
   cudaFree(ctx->d_adj_dk);
   cudaFree(ctx->d_adj_mom);
@@ -1832,22 +1829,6 @@ __global__ void adj_moments_kernel(const double *x, const double *y, const int32
   }
 }
 
-/* lambda at the end of the run: dL/dx = (2 x + 2 w mean(x)) / N, same in y,
- * with coef[3 v .. 3 v + 2] = (2 w mean(x) / N, 2 w mean(y) / N, 1 / N) of
- * the particle's variant */
-__global__ void adj_seed_kernel(const double *x, const double *y, const int32_t *lost, long n, double *lam,
-                                const long *offsets, int nv, const double *coef) {
-  for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
-    const bool act = lost[i] < 0;
-    const double *c = coef + 3 * adj_variant(offsets, nv, i);
-    lam[i] = act ? 2 * x[i] * c[2] + c[0] : 0;
-    lam[n + i] = 0;
-    lam[2 * n + i] = act ? 2 * y[i] * c[2] + c[1] : 0;
-    lam[3 * n + i] = 0;
-    lam[4 * n + i] = 0;
-  }
-}
-
 /* L_v = mean(x^2 + y^2) + w (mean(x)^2 + mean(y)^2) over the survivors of
  * each variant (nv = 1 and offsets = null: the whole beam); mom receives
  * (L, mean x, mean y, count) per variant */
@@ -1914,8 +1895,9 @@ static int param_derivative(const trk_elem *e, double Po, double *dk3) {
   return TRK_OK;
 }
 
-/* d(Fx, Fy)/dK1 and d(Fx, Fy)/dK2 of a CSBEND's field expansion, as 4 x 121
- * doubles (Fx, Fy per unit K1, then per unit K2).  The expansion is linear
+/* d(Fx, Fy)/dK1 and d(Fx, Fy)/dK2 of a CSBEND's field expansion, packed as
+ * adj_dfield reads them: the nonzero entries i + j <= 4 of Fy and Fx per unit
+ * K1, then per unit K2.  The expansion is linear
  * in b[] (trk_csbend_field_table), and b1 = K1 (L/ANGLE) (1+FSE+FSE_Q)/
  * (1+FSE+FSE_D), b2 = K2 (L/ANGLE) (1+FSE)/(1+FSE+FSE_D), odd b's flipped
  * for ANGLE < 0 (compile_bend): the tables are the expansion of those unit
@@ -1937,11 +1919,15 @@ static int csbend_field_derivatives(const trk_elem *e, double *out) {
     if (order != 4)
       return trk_set_error(TRK_ERR_UNSUPPORTED, "CSBEND gradients need EXPANSION_ORDER 0 or 4");
     int eo1, hn, hs;
-    double *Fx = out + 242 * q, *Fy = Fx + 121;
+    double Fx[121] = {0}, Fy[121] = {0};
     if (trk_csbend_field_table(b, c, 1 / rho, (int)TRK_P(e, CSBEND_NONLINEAR), order, Fx, Fy, &eo1, &hn, &hs))
       return trk_set_error(TRK_ERR_UNSUPPORTED, "CSBEND expansion order too high");
     Fx[0] = 0;
     Fy[0] = 0;
+    for (int k : {q ? 22 : 11, 2, 13, 24, 4})
+      *out++ = Fy[k];
+    for (int k : {q ? 12 : 1, 3, 14})
+      *out++ = Fx[k];
   }
   return TRK_OK;
 }
@@ -1989,6 +1975,7 @@ static int adjoint_run(trk_context *ctx, const trk_lattice *const *lattices, int
   }
   std::vector<int> op_dfield(std::max(nops, 1), -1);
   std::vector<double> dfield;
+  std::vector<const trk_elem *> dfield_elem; /* the bend each table was formed for */
   for (int k = 0; k < nops; k++) {
     const trk_op &op = c.ops[k];
     switch (op.kind) {
@@ -2028,10 +2015,21 @@ static int adjoint_run(trk_context *ctx, const trk_lattice *const *lattices, int
             return trk_set_error(TRK_ERR_UNSUPPORTED, "element %d: CSBEND gradients need the variants to share "
                                  "L, ANGLE, FSE* and the expansion settings", op.elem);
       op_param[k] = pe;
-      op_dfield[k] = (int)dfield.size();
-      dfield.resize(dfield.size() + 4 * 121);
-      if ((rc = csbend_field_derivatives(e0, dfield.data() + op_dfield[k])))
-        return rc;
+      /* one table for bends that share everything it depends on */
+      for (size_t m = 0; m < dfield_elem.size() && op_dfield[k] < 0; m++) {
+        bool eq = true;
+        for (int q : same)
+          eq = eq && dfield_elem[m]->p[q] == e0->p[q];
+        if (eq)
+          op_dfield[k] = (int)m * TRK_DFIELD_LEN;
+      }
+      if (op_dfield[k] < 0) {
+        op_dfield[k] = (int)dfield.size();
+        dfield.resize(dfield.size() + TRK_DFIELD_LEN);
+        dfield_elem.push_back(e0);
+        if ((rc = csbend_field_derivatives(e0, dfield.data() + op_dfield[k])))
+          return rc;
+      }
     } else if (pe >= 0) {
       if (op.kind != OPK_MULT1)
         return trk_set_error(TRK_ERR_UNSUPPORTED, "element %d: gradients need a single-order multipole", op.elem);
@@ -2043,9 +2041,7 @@ static int adjoint_run(trk_context *ctx, const trk_lattice *const *lattices, int
   }
   const long np = ctx->np, T = run->n_passes;
   const size_t n_grad_all = (size_t)n_params * nv;
-  if ((rc = ensure(&ctx->d_adj_ck, ctx->adj_ck_cap, (size_t)T * 4 * np)) ||
-      (rc = ensure(&ctx->d_adj_entry, ctx->adj_entry_cap, (size_t)std::max(nops, 1) * 4 * np)) ||
-      (rc = ensure(&ctx->d_adj_lam, ctx->adj_lam_cap, (size_t)5 * np)) ||
+  if ((rc = ensure(&ctx->d_adj_ck, ctx->adj_ck_cap, (size_t)std::max(grad ? T - 1 : 0, 1L) * 4 * np)) ||
       (rc = ensure(&ctx->d_adj_grad, ctx->adj_grad_cap, std::max<size_t>(n_grad_all, 1))) ||
       (rc = ensure(&ctx->d_adj_param, ctx->adj_param_cap, op_param.size())) ||
       (rc = ensure(&ctx->d_adj_dk, ctx->adj_dk_cap, op_dk.size())) ||
@@ -2062,7 +2058,7 @@ static int adjoint_run(trk_context *ctx, const trk_lattice *const *lattices, int
   CUDA_TRY(cudaMemcpyAsync(ctx->d_adj_dk, op_dk.data(), sizeof(double) * op_dk.size(), cudaMemcpyHostToDevice,
                            ctx->stream));
 
-  /* forward, one pass per launch, the beam at the start of every pass kept */
+  /* forward, one pass per launch, the beam at the end of every pass but the last kept */
   const long p0 = run->pass_offset;
   const long fresh = ctx->passes_done == 0 ? p0 : -1;
   if (fresh >= 0)
@@ -2076,9 +2072,6 @@ static int adjoint_run(trk_context *ctx, const trk_lattice *const *lattices, int
   const long *d_off = ensemble ? ctx->d_ens_offsets : nullptr;
   const int shape = trk_default_variant(true, c);
   for (long t = 0; t < T; t++) {
-    for (int q = 0; q < 4; q++)
-      CUDA_TRY(cudaMemcpyAsync(ctx->d_adj_ck + ((size_t)t * 4 + q) * np, ctx->d_cols + (size_t)q * ctx->cap,
-                               sizeof(double) * np, cudaMemcpyDeviceToDevice, ctx->stream));
     ta.pass_begin = p0 + t;
     ta.pass_end = p0 + t + 1;
     if (nops > 0) {
@@ -2088,6 +2081,9 @@ static int adjoint_run(trk_context *ctx, const trk_lattice *const *lattices, int
       else
         trk_fast::launch_track(ta, shape, trk_lean_flavor(c), np, ctx->sm_count * 256, ctx->stream);
     }
+    for (int q = 0; q < 4 && grad && t < T - 1; q++)
+      CUDA_TRY(cudaMemcpyAsync(ctx->d_adj_ck + ((size_t)t * 4 + q) * np, ctx->d_cols + (size_t)q * ctx->cap,
+                               sizeof(double) * np, cudaMemcpyDeviceToDevice, ctx->stream));
   }
   CUDA_TRY(cudaGetLastError());
   ctx->passes_done += T;
@@ -2100,8 +2096,7 @@ static int adjoint_run(trk_context *ctx, const trk_lattice *const *lattices, int
   if (!grad)
     return TRK_OK;
 
-  /* reverse: seed, then per pass (last first) record the element entry
-   * states from the pass checkpoint and sweep the elements backwards */
+  /* reverse: every pass backwards in one launch, from the final beam and the checkpoints */
   std::vector<double> coef(3 * (size_t)nv);
   for (int v = 0; v < nv; v++) {
     const double cnt = mom[4 * v + 3];
@@ -2113,12 +2108,11 @@ static int adjoint_run(trk_context *ctx, const trk_lattice *const *lattices, int
    * contents are no longer needed */
   CUDA_TRY(cudaMemcpyAsync(ctx->d_adj_mom, coef.data(), sizeof(double) * coef.size(), cudaMemcpyHostToDevice,
                            ctx->stream));
-  adj_seed_kernel<<<std::min(grid_for(ctx, np, 256), 1184), 256, 0, ctx->stream>>>(
-    ctx->d_cols, ctx->d_cols + 2 * ctx->cap, ctx->d_lost_pass, np, ctx->d_adj_lam, d_off, nv, ctx->d_adj_mom);
   CUDA_TRY(cudaMemsetAsync(ctx->d_adj_grad, 0, sizeof(double) * std::max<size_t>(n_grad_all, 1), ctx->stream));
   AdjArgs g;
-  g.entry = ctx->d_adj_entry;
-  g.lam = ctx->d_adj_lam;
+  g.ck = ctx->d_adj_ck;
+  g.coef = ctx->d_adj_mom;
+  g.n_passes = T;
   g.grad = ctx->d_adj_grad;
   g.op_param = ctx->d_adj_param;
   g.op_dk = ctx->d_adj_dk;
@@ -2131,11 +2125,7 @@ static int adjoint_run(trk_context *ctx, const trk_lattice *const *lattices, int
     ta.ens_variants = nv;
     ta.ens_ops = nops;
   }
-  for (long t = T - 1; t >= 0; t--) {
-    g.ck = ctx->d_adj_ck + (size_t)t * 4 * np;
-    trk_fast::launch_adjoint_record(ta, g, ctx->stream);
-    trk_fast::launch_adjoint_reverse(ta, g, ctx->stream);
-  }
+  trk_fast::launch_adjoint_reverse(ta, g, ctx->stream);
   CUDA_TRY(cudaGetLastError());
   CUDA_TRY(cudaMemcpyAsync(grad, ctx->d_adj_grad, sizeof(double) * n_grad_all, cudaMemcpyDeviceToHost,
                            ctx->stream));

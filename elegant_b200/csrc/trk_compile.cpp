@@ -1045,8 +1045,9 @@ int trk_compile(const trk_lattice *l, double Po, CompiledLattice &out) {
       else if (plain && op.i[2] == 1 && op.i[3] == 5) {
         op.kind = OPK_CFBEND;
         out.has_cfbend = true;
-        const double *Fy = out.field.data() + op.i[4] + 121;
-        if (Fy[2 * 11] == 0 && Fy[3 * 11] == 0 && Fy[4 * 11] == 0)
+        const double *Fx = out.field.data() + op.i[4], *Fy = Fx + 121;
+        if (Fy[2 * 11] == 0 && Fy[3 * 11] == 0 && Fy[4 * 11] == 0 && Fx[11 + 1] == 0 && Fx[2 * 11 + 1] == 0 &&
+            Fx[3 * 11 + 1] == 0)
           op.i[7] |= BF_LINEAR;
       }
       /* the merged bodies take |q| up to 2^-6: inside a slice the design

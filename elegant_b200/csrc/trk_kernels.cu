@@ -2224,7 +2224,7 @@ __device__ __forceinline__ void op_dipole_fast2(const trk_op *__restrict__ op, P
  * Bound by FP64 issue and by the length of the substep's chain (13 of its 17
  * operations).  Measured against the checked bodies alone, ms per turn: FODO
  * ring with RF and wake, 1e6 particles, 11.4 -> 7.6; achromat ring, 2e6, 250
- * -> 169; FODO ring, 1e4 particles, 0.67 -> 0.41; dynamic-aperture grids over
+ * -> 158; FODO ring, 1e4 particles, 0.67 -> 0.41; dynamic-aperture grids over
  * 24 seeds, where the checked bodies divide for the aperture in every slice,
  * 101 -> 46 for 32 turns. */
 
@@ -2419,7 +2419,7 @@ __device__ __forceinline__ bool dipole_merged(const double *__restrict__ d, int 
 }
 
 /* OPK_CFBEND: the same with kicks that change py.  The field as in cf_fields;
- * LIN: K1 only, the midplane field linear in x. */
+ * LIN: K1 only, the midplane field linear in x and its slope constant. */
 template <bool LIN>
 __device__ __forceinline__ bool cfbend_merged(const double *__restrict__ d, const double *__restrict__ fxy, int nSlices,
                                               Part &p, const trk_aperture *__restrict__ ap) {
@@ -2459,7 +2459,9 @@ __device__ __forceinline__ bool cfbend_merged(const double *__restrict__ d, cons
                 CF_T(Ty, 0, 0));                                                                             \
     const double p2 = fma(fma(CF_T(Ty, 2, 2), X, CF_T(Ty, 1, 2)), X, CF_T(Ty, 0, 2));                        \
     const double fy = fma(y2, fma(y2, CF_T(Ty, 0, 4), p2), p0);                                              \
-    const double q1 = fma(fma(fma(CF_T(Tx, 3, 1), X, CF_T(Tx, 2, 1)), X, CF_T(Tx, 1, 1)), X, CF_T(Tx, 0, 1)); \
+    const double q1 =                                                                                        \
+      LIN ? CF_T(Tx, 0, 1)                                                                                   \
+          : fma(fma(fma(CF_T(Tx, 3, 1), X, CF_T(Tx, 2, 1)), X, CF_T(Tx, 1, 1)), X, CF_T(Tx, 0, 1));          \
     const double q3 = fma(CF_T(Tx, 1, 3), X, CF_T(Tx, 0, 3));                                                \
     const double wk = (K) * R;                                                                               \
     px = fma(-wk, fy, px);                                                                                   \
@@ -3439,231 +3441,162 @@ __global__ void matrix_kernel(TrackArgs a, const double *__restrict__ m, int ord
 
 #if TRK_FAST
 /* ------------------------------------------------------------- adjoint
- * Reverse mode through the fast build's element maps.  The forward values
- * inside an element are recomputed from its entry state (recorded per pass
- * by adj_record_kernel) and the chain rule is applied backwards, operation
- * by operation, to the adjoint (lambda) of x, x', y, y', delta.  Parameter
- * sensitivities of the kick strengths are summed per warp and added to the
- * gradient with one atomic per warp and element. */
-#define TRK_ADJ_MAX_KICKS 48  /* multipole: slices * 3 kicks */
-#define TRK_ADJ_MAX_STEPS 128 /* dipole: slices * 4 substeps */
+ * Reverse mode through the fast build's element maps, in the momenta of the
+ * merged bodies (divided by the total momentum).  The maps are inverted
+ * exactly, substep by substep: a kick leaves the position it was taken at, a
+ * drift the momenta (in a bend, a rotation).  So the sweep needs no recorded
+ * states inside a pass: it starts from the beam at the end of the pass (the
+ * next pass's checkpoint) and carries the particle and its adjoint (lambda of
+ * x, x', y, y') back through the elements together.  One thread takes one
+ * particle through all passes of the run.  Parameter sensitivities of the
+ * kick strengths are summed per warp and added to the gradient with one
+ * atomic per warp and element.  delta has no adjoint: nothing on this path
+ * changes it.
+ *
+ * Bound by FP64 issue and the length of a substep's chain (60 % of the FP64
+ * pipe with every SM full): about 43 operations per substep of a dipole and
+ * 25 more for the K1 and K2 sensitivities of its kick.  Measured on the FODO
+ * ring with sextupoles, 1e5 particles, per turn, forward pass included: 4.8
+ * ms; recording every element's entry state and every substep's in local
+ * memory took 14.5 ms and 9 GB of memory traffic.  (128, 4) with 122
+ * registers: (128, 6) with 80 is 1 % slower at 1e5 particles and more, 7 %
+ * below a block per SM. */
 
-/* (sx, sy) = (qx, qy) / sqrt((1+delta)^2 - qx^2 - qy^2): adds the adjoint of
- * qx, qy, delta given that of sx, sy */
-__device__ __forceinline__ void adj_m2s(double qx, double qy, double opd, double lsx, double lsy, double &lqx,
-                                        double &lqy, double &ldp) {
-  const double g = rsqrt_fast(opd * opd - qx * qx - qy * qy);
-  const double g3 = g * g * g;
-  lqx += lsx * (g + qx * qx * g3) + lsy * (qx * qy * g3);
-  lqy += lsx * (qx * qy * g3) + lsy * (g + qy * qy * g3);
-  ldp -= (lsx * qx + lsy * qy) * opd * g3;
+/* 1/sqrt(1 - z) and sqrt(1 - z) = (1 - z)/sqrt(1 - z) for any z < 1 */
+__device__ __forceinline__ double sec_any(double z) {
+  if ((unsigned)__double2hiint(z) < TRK_Z_HI)
+    return 1 + sec_m1(z);
+  return rsqrt_fast(1 - z);
 }
 
-/* (qx, qy) = (1+delta) (xp, yp) / sqrt(1 + xp^2 + yp^2): adjoint of xp, yp,
- * delta given that of qx, qy */
-__device__ __forceinline__ void adj_s2m(double xp, double yp, double opd, double lqx, double lqy, double &lxp,
-                                        double &lyp, double &ldp) {
-  const double rs = rsqrt_fast(fma(yp, yp, fma(xp, xp, 1.0)));
-  const double rs3 = rs * rs * rs;
-  lxp += lqx * opd * (rs - xp * xp * rs3) - lqy * opd * xp * yp * rs3;
-  lyp += lqy * opd * (rs - yp * yp * rs3) - lqx * opd * xp * yp * rs3;
-  ldp += (lqx * xp + lqy * yp) * rs;
+/* the particle and its adjoint inside an element: momenta px, py */
+struct AdjState {
+  double x, px, y, py;
+  double lx, lpx, ly, lpy;
+};
+
+/* element exit: slopes to momenta, and the adjoint of (x', y') = (px, py)/pz */
+__device__ __forceinline__ void adj_enter(AdjState &q) {
+  const double xp = q.px, yp = q.py;
+  const double ss = fma(yp, yp, fma(xp, xp, 1.0)), r = rsqrt_fast(ss), sec = ss * r;
+  q.px = xp * r;
+  q.py = yp * r;
+  const double t = (sec * sec * sec) * fma(q.px, q.lpx, q.py * q.lpy);
+  q.lpx = fma(sec, q.lpx, q.px * t);
+  q.lpy = fma(sec, q.lpy, q.py * t);
 }
 
-/* normal multipole field of order 1..3 with the fast build's coefficients:
- * kick qx -= K Fy, qy += K Fx, and the partial derivatives */
-__device__ __forceinline__ void mult_field(int order, double x, double y, double &Fy, double &Fx, double &Fyx,
-                                           double &Fyy, double &Fxx, double &Fxy) {
-  if (order == 1) {
-    Fy = x;
-    Fx = y;
-    Fyx = 1;
-    Fyy = 0;
-    Fxx = 0;
-    Fxy = 1;
-  } else if (order == 2) {
-    Fy = 0.5 * (x * x - y * y);
+/* element entry: momenta to slopes, and the adjoint of px = x'/sqrt(1 + x'^2 + y'^2) */
+__device__ __forceinline__ void adj_leave(AdjState &q) {
+  const double z = fma(q.px, q.px, q.py * q.py), sec = sec_any(z), pz = fma(-z, sec, sec);
+  const double t = fma(q.px, q.lpx, q.py * q.lpy);
+  q.lpx = pz * fma(-q.px, t, q.lpx);
+  q.lpy = pz * fma(-q.py, t, q.lpy);
+  q.px *= sec;
+  q.py *= sec;
+}
+
+/* a straight drift: x += px l, y += py l, l = L/pz */
+__device__ __forceinline__ void adj_straight(AdjState &q, double L) {
+  const double sec = sec_any(fma(q.px, q.px, q.py * q.py)), l = L * sec;
+  q.x = fma(-q.px, l, q.x);
+  q.y = fma(-q.py, l, q.y);
+  const double t = (l * sec * sec) * fma(q.px, q.lx, q.py * q.ly);
+  q.lpx = fma(l, q.lx, fma(q.px, t, q.lpx));
+  q.lpy = fma(l, q.ly, fma(q.py, t, q.lpy));
+}
+
+/* a multipole kick px -= K Fy, py += K Fx; returns -Fy lpx + Fx lpy, the
+ * sensitivity to K */
+template <int ORDER> __device__ __forceinline__ double adj_kick(AdjState &q, double K) {
+  double Fy, Fx;
+  const double lpx = q.lpx, lpy = q.lpy;
+  if (ORDER == 1) {
+    Fy = q.x;
+    Fx = q.y;
+    q.lx = fma(-K, lpx, q.lx);
+    q.ly = fma(K, lpy, q.ly);
+  } else if (ORDER == 2) {
+    const double x = q.x, y = q.y;
+    Fy = 0.5 * fma(x, x, -y * y);
     Fx = x * y;
-    Fyx = x;
-    Fyy = -y;
-    Fxx = y;
-    Fxy = x;
+    q.lx = fma(K, fma(-x, lpx, y * lpy), q.lx);
+    q.ly = fma(K, fma(y, lpx, x * lpy), q.ly);
   } else {
-    const double x2 = x * x, y2 = y * y;
-    Fy = (x2 * x - 3 * x * y2) * (1.0 / 6);
-    Fx = (3 * x2 * y - y2 * y) * (1.0 / 6);
-    Fyx = 0.5 * (x2 - y2);
-    Fyy = -x * y;
-    Fxx = x * y;
-    Fxy = 0.5 * (x2 - y2);
+    const double x = q.x, y = q.y, x2 = x * x, y2 = y * y;
+    Fy = fma(-3.0, y2, x2) * x * (1.0 / 6);
+    Fx = fma(3.0, x2, -y2) * y * (1.0 / 6);
+    const double a = 0.5 * (x2 - y2), b = x * y;
+    q.lx = fma(K, fma(-a, lpx, b * lpy), q.lx);
+    q.ly = fma(K, fma(b, lpx, a * lpy), q.ly);
   }
+  q.px = fma(K, Fy, q.px);
+  q.py = fma(-K, Fx, q.py);
+  return fma(-Fy, lpx, Fx * lpy);
 }
 
-/* adjoint of op_mult1_fast (the body of mult_body_fast); returns the
- * sensitivity of the particle's contribution to the element's parameter */
-__device__ double adj_mult1(const trk_op *__restrict__ op, const double *__restrict__ dk, double x, double xp,
-                            double y, double yp, double dp, double &lx, double &lxp, double &ly, double &lyp,
-                            double &ldp) {
+/* OPK_MULT1 backwards; returns the sensitivity to the element's parameter */
+template <int ORDER>
+__device__ __forceinline__ double adj_mult1(const trk_op *__restrict__ op, const double *__restrict__ dk, double opd,
+                                            AdjState &q) {
   const double *d = op->d;
   const int n_parts = __ldg(&op->i[0]);
-  const int order = __ldg(&op->i[4]) & 0xff;
-  const double opd = 1 + dp, opd2 = opd * opd;
-  double KX[TRK_ADJ_MAX_KICKS], KY[TRK_ADJ_MAX_KICKS], QX[TRK_ADJ_MAX_KICKS], QY[TRK_ADJ_MAX_KICKS];
-  const double r = opd * rsqrt_fast(fma(yp, yp, fma(xp, xp, 1.0)));
-  double qx = xp * r, qy = yp * r, sx = xp, sy = yp;
-  int nk = 0;
-  for (int i_kick = 0; i_kick < n_parts; i_kick++)
-    for (int step = 0; step < 4; step++) {
-      const double dsh = __ldg(&d[MD_DSH + step]);
-      x = fma(sx, dsh, x);
-      y = fma(sy, dsh, y);
-      if (step == 3)
-        break;
-      const double K = __ldg(&d[MD_KQ + step * 3]);
-      double Fy, Fx, a, b, c, e;
-      mult_field(order, x, y, Fy, Fx, a, b, c, e);
-      qx = fma(-K, Fy, qx);
-      qy = fma(K, Fx, qy);
-      const double rr = rsqrt_fast(opd2 - qx * qx - qy * qy);
-      sx = qx * rr;
-      sy = qy * rr;
-      KX[nk] = x;
-      KY[nk] = y;
-      QX[nk] = qx;
-      QY[nk] = qy;
-      nk++;
-    }
-  /* exit slopes from the final momenta */
-  double lqx = 0, lqy = 0, lsx = 0, lsy = 0, sens = 0;
-  adj_m2s(qx, qy, opd, lxp, lyp, lqx, lqy, ldp);
-  for (int i_kick = n_parts - 1; i_kick >= 0; i_kick--)
-    for (int step = 3; step >= 0; step--) {
-      if (step < 3) {
-        nk--;
-        adj_m2s(QX[nk], QY[nk], opd, lsx, lsy, lqx, lqy, ldp);
-        lsx = lsy = 0;
-        const double K = __ldg(&d[MD_KQ + step * 3]);
-        double Fy, Fx, Fyx, Fyy, Fxx, Fxy;
-        mult_field(order, KX[nk], KY[nk], Fy, Fx, Fyx, Fyy, Fxx, Fxy);
-        lx += K * (-Fyx * lqx + Fxx * lqy);
-        ly += K * (-Fyy * lqx + Fxy * lqy);
-        sens += (-Fy * lqx + Fx * lqy) * __ldg(&dk[step]);
-      }
-      const double dsh = __ldg(&d[MD_DSH + step]);
-      lsx += dsh * lx;
-      lsy += dsh * ly;
-    }
-  /* entry: the first drift used the incoming slopes; the momenta came from them */
-  double lxp_in = lsx, lyp_in = lsy;
-  adj_s2m(xp, yp, opd, lqx, lqy, lxp_in, lyp_in, ldp);
-  lxp = lxp_in;
-  lyp = lyp_in;
-  return sens;
+  const double iopd = rcp_fast(opd);
+  const double l0 = __ldg(&d[MD_DSH]), l1 = __ldg(&d[MD_DSH + 1]);
+  const double ka = __ldg(&d[MD_KQ]) * iopd, kb = __ldg(&d[MD_KQ + 3]) * iopd;
+  double sa = 0, sb = 0;
+  adj_enter(q);
+  for (int i = n_parts; i > 0; i--) {
+    adj_straight(q, i < n_parts ? 2 * l0 : l0);
+    sa += adj_kick<ORDER>(q, ka);
+    adj_straight(q, l1);
+    sb += adj_kick<ORDER>(q, kb);
+    adj_straight(q, l1);
+    sa += adj_kick<ORDER>(q, ka);
+  }
+  adj_straight(q, l0);
+  adj_leave(q);
+  return iopd * fma(__ldg(&dk[0]), sa, __ldg(&dk[1]) * sb);
 }
 
-/* adjoint of op_dipole_fast (bend_dipole_fast / dipole_slice) */
-/* The adjoint of the pure-dipole body; with dk (the bend's field
- * derivative tables, dF/dK1 at dk and dF/dK2 at dk + 242) it also returns
- * the sensitivities to the bend's K1 and K2 at K1 = K2 = 0: each kick
- * QX -= w Fy, QY += w Fx changes by -w dFy, +w dFx per unit K, weighted by
- * the adjoints of QX and QY after the kick (QY's running adjoint collects
- * the later drifts' shares as the sweep goes back). */
-__device__ void adj_dipole(const trk_op *__restrict__ op, double x, double xp, double y, double yp, double dp,
-                           double &lx, double &lxp, double &ly, double &lyp, double &ldp,
-                           const double *__restrict__ dk = nullptr, double *sk = nullptr) {
-  const double *d = op->d;
-  const int nSlices = __ldg(&op->i[0]);
-  const double rho0 = __ldg(&d[BD_RHO0]);
-  const double opd = 1 + dp;
-  const double rs = rsqrt_fast(fma(yp, yp, fma(xp, xp, 1.0)));
-  const double QY = yp * opd * rs;
-  const double f2 = opd * opd - QY * QY;
-  double X = x, Q = xp * opd * rs, F = 0;
-  double SX[TRK_ADJ_MAX_STEPS], SQ[TRK_ADJ_MAX_STEPS], SF[TRK_ADJ_MAX_STEPS];
-  int m = 0;
-  for (int i = 0; i < nSlices; i++)
-    for (int j = 0; j < 4; j++) {
-      SX[m] = X;
-      SQ[m] = Q;
-      SF[m] = F;
-      m++;
-      const double sa = __ldg(&d[BD_SA + j]), ca = __ldg(&d[BD_CA + j]), omc = __ldg(&d[BD_OMC + j]);
-      const double fc = sqrt_nan(fma(-Q, Q, f2));
-      const double saq = sa * Q;
-      const double u = div_fast(rho0 + X, fma(ca, fc, -saq));
-      Q = fma(sa, fc, ca * Q);
-      F = fma(u, sa, F);
-      X = fma(u, fma(omc, fc, saq), X);
-      if (j < 3)
-        Q = fma(-__ldg(&d[BD_C2 + j]), X, Q - __ldg(&d[BD_C1 + j]));
-    }
-  const int nsteps = m;
-  /* exit: x = X, y = y0 + QY F, (xp, yp) = (Q, QY) / sqrt(opd^2 - Q^2 - QY^2) */
-  double lX = lx, lQ = 0, lQY = 0, lopd = 0, lF = QY * ly, lf2 = 0;
-  {
-    const double g = rsqrt_fast(opd * opd - Q * Q - QY * QY);
-    const double g3 = g * g * g;
-    lQ += lxp * (g + Q * Q * g3) + lyp * Q * QY * g3;
-    lQY += lyp * (g + QY * QY * g3) + lxp * Q * QY * g3;
-    lopd -= (lxp * Q + lyp * QY) * opd * g3;
-  }
-  double sk1 = 0, sk2 = 0;
-  for (int i = nSlices - 1; i >= 0; i--)
-    for (int j = 3; j >= 0; j--) {
-      if (j < 3) {
-        const double c2 = __ldg(&d[BD_C2 + j]);
-        if (dk) {
-          /* the kick at the end of drift j: position X1, Y1 = y + QY F1 */
-          const double X1 = m < nsteps ? SX[m] : X, Y1 = fma(QY, m < nsteps ? SF[m] : F, y);
-          const double w = fma(c2, X1, __ldg(&d[BD_C1 + j]));
-          double dFx, dFy;
-          cf_fields(dk, dk + 121, X1, Y1, dFx, dFy);
-          sk1 += w * (lQY * dFx - lQ * dFy);
-          cf_fields(dk + 242, dk + 363, X1, Y1, dFx, dFy);
-          sk2 += w * (lQY * dFx - lQ * dFy);
-        }
-        lX -= c2 * lQ;
-      }
-      m--;
-      const double Xs = SX[m], Qs = SQ[m];
-      const double sa = __ldg(&d[BD_SA + j]), ca = __ldg(&d[BD_CA + j]), omc = __ldg(&d[BD_OMC + j]);
-      const double fc = sqrt_nan(fma(-Qs, Qs, f2));
-      const double saq = sa * Qs;
-      const double fcosi = fma(ca, fc, -saq);
-      const double u = div_fast(rho0 + Xs, fcosi);
-      const double lu = lF * sa + lX * fma(omc, fc, saq);
-      double lfc = lQ * sa + lX * u * omc;
-      double lsaq = lX * u;
-      double lQs = lQ * ca;
-      double lXs = lX;
-      const double lfcosi = -lu * u / fcosi;
-      lXs += lu / fcosi;
-      lfc += ca * lfcosi;
-      lsaq -= lfcosi;
-      lQs += sa * lsaq;
-      const double lu2 = lfc / (2 * fc);
-      lf2 += lu2;
-      /* this drift's share of QY's adjoint: Y grows by QY u sa, f2 holds -QY^2 */
-      lQY += ly * u * sa - 2 * QY * lu2;
-      lQs -= 2 * Qs * lu2;
-      lX = lXs;
-      lQ = lQs;
-    }
-  lopd += 2 * opd * lf2;
-  if (sk) {
-    sk[0] = sk1;
-    sk[1] = sk2;
-  }
-  /* entry: X = x, (Q, QY) = opd (xp, yp) / sqrt(1 + xp^2 + yp^2) */
-  const double rs3 = rs * rs * rs;
-  lx = lX;
-  lxp = lQ * opd * (rs - xp * xp * rs3) - lQY * opd * xp * yp * rs3;
-  lyp = lQY * opd * (rs - yp * yp * rs3) - lQ * opd * xp * yp * rs3;
-  lopd += (lQ * xp + lQY * yp) * rs;
-  ldp += lopd;
+/* A bend's drift through the angle a: (px, pz) rotates, R' = R pz/pz', Y' = Y +
+ * py D with D = R sin(a)/pz'.  From R' and the derivatives of pz, pz':
+ *   dpx'/dpx = pz'/pz, dpx'/dpy = -sin(a) py/pz,
+ *   dR'/dR = pz/pz',   dR'/dpx = M (1 - py^2),  dR'/dpy = M px py,
+ *   dD/dR = sin(a)/pz', dD/dpx = M px',          dD/dpy = M cos(a) py,
+ * with M = sin(a) R/(pz pz'^2). */
+__device__ __forceinline__ void adj_rotate(AdjState &q, double rho0, double sa, double ca, double omc) {
+  const double py2 = q.py * q.py;
+  const double z1 = fma(q.px, q.px, py2), sec1 = sec_any(z1), pz1 = fma(-z1, sec1, sec1);
+  const double px1 = q.px, R1 = rho0 + q.x;
+  q.px = fma(ca, px1, -(sa * pz1));
+  const double z = fma(q.px, q.px, py2), sec = sec_any(z), pz = fma(-z, sec, sec);
+  q.x = fma(R1 * sec, fma(omc, pz1, -(sa * px1)), q.x);
+  const double a1 = sa * sec1, D = (rho0 + q.x) * a1, M = D * (sec * sec1);
+  q.y = fma(-q.py, D, q.y);
+  const double lR1 = q.lx, lpx1 = q.lpx, lD = q.ly * q.py;
+  q.lx = fma(lR1, pz * sec1, lD * a1);
+  q.lpx = fma(lpx1, pz1 * sec, M * fma(1 - py2, lR1, lD * px1));
+  q.lpy = fma(q.ly, D, fma(q.py, fma(M, fma(lR1, q.px, lD * ca), -(lpx1 * (sa * sec))), q.lpy));
 }
 
-#define TRK_ADJ_MAX_SLICES 32 /* combined-function bend: slices */
+/* d(Fx, Fy)/dK1 and dK2 of a bend's field expansion at (x, y) times (lpy,
+ * -lpx).  On the midplane the unit fields are Fy = x and x^2/2 exactly, and
+ * Fx's first order in y is their derivative, so of the entries i + j <= 4 only
+ * Fy's 10 (K2: 20), 02, 12, 22, 04 and Fx's 01 (K2: 11), 03, 13 are not zero:
+ * packed in that order, K1 then K2. */
+__device__ __forceinline__ void adj_dfield(const double *__restrict__ t, double x, double y, double lpx, double lpy,
+                                           double w, double *sk) {
+  const double y2 = y * y;
+#pragma unroll
+  for (int m = 0; m < 2; m++, t += TRK_DFIELD_LEN / 2) {
+    const double mid = m ? __ldg(&t[0]) * x : __ldg(&t[0]), slope = m ? __ldg(&t[5]) * x : __ldg(&t[5]);
+    const double p2 = fma(fma(__ldg(&t[3]), x, __ldg(&t[2])), x, __ldg(&t[1]));
+    const double dFy = fma(mid, x, y2 * fma(y2, __ldg(&t[4]), p2));
+    const double dFx = y * fma(y2, fma(__ldg(&t[7]), x, __ldg(&t[6])), slope);
+    sk[m] = fma(w, fma(-lpx, dFy, lpy * dFx), sk[m]);
+  }
+}
 
 /* partial derivatives of the cf_fields expansion at (x, y) */
 #define CF_T(T, i, j) __ldg(&(T)[(i) * 11 + (j)])
@@ -3686,193 +3619,61 @@ __device__ __forceinline__ void cf_fields_d(const double *__restrict__ Fx_xy, co
 }
 #undef CF_T
 
-/* one drift substep j of cf_slice (no path length) */
-__device__ __forceinline__ void cf_drift(const double *__restrict__ d, int j, double rho0, double opd2, double &X,
-                                         double &QX, double &Y, const double QY) {
-  const double fc = sqrt_nan(fma(-QX, QX, fma(-QY, QY, opd2)));
-  const double sa = __ldg(&d[BD_SA + j]), ca = __ldg(&d[BD_CA + j]);
-  const double saq = sa * QX;
-  const double u = div_fast(rho0 + X, fma(ca, fc, -saq));
-  QX = fma(sa, fc, ca * QX);
-  Y = fma(QY, u * sa, Y);
-  X = fma(u, fma(__ldg(&d[BD_OMC + j]), fc, saq), X);
+/* the kick at a drift's start or end: px -= w Fy, py += w Fx, w = k R (CF: the
+ * bend's field expansion; a pure dipole's Fx = 0, Fy = 1).  With dk, adds the
+ * sensitivities to the bend's K1 and K2 to sk. */
+template <bool CF>
+__device__ __forceinline__ void adj_bend_kick(AdjState &q, double k, double rho0, const double *__restrict__ fx,
+                                              const double *__restrict__ dk, double *sk) {
+  const double w = k * (rho0 + q.x), lpx = q.lpx, lpy = q.lpy;
+  if (dk)
+    adj_dfield(dk, q.x, q.y, lpx, lpy, w, sk);
+  if (CF) {
+    double Fx, Fy, Fyx, Fyy, Fxx, Fxy;
+    cf_fields(fx, fx + 121, q.x, q.y, Fx, Fy);
+    cf_fields_d(fx, fx + 121, q.x, q.y, Fyx, Fyy, Fxx, Fxy);
+    q.px = fma(w, Fy, q.px);
+    q.py = fma(-w, Fx, q.py);
+    q.lx = fma(k, fma(-lpx, Fy, lpy * Fx), fma(w, fma(-lpx, Fyx, lpy * Fxx), q.lx));
+    q.ly = fma(w, fma(-lpx, Fyy, lpy * Fxy), q.ly);
+  } else {
+    q.px += w;
+    q.lx = fma(-k, lpx, q.lx);
+  }
 }
 
-/* adjoint of op_cfbend_fast (bend_cf_fast / cf_slice): the entry state of
- * every slice is kept, and each slice's four substeps are recomputed from it
- * while the slices are reversed */
-__device__ void adj_cfbend(const trk_op *__restrict__ op, const double *__restrict__ field, double x, double xp,
-                           double y, double yp, double dp, double &lx, double &lxp, double &ly, double &lyp,
-                           double &ldp, const double *__restrict__ dk = nullptr, double *sk = nullptr) {
+/* OPK_DIPOLE and OPK_CFBEND backwards */
+template <bool CF>
+__device__ __forceinline__ void adj_bend(const trk_op *__restrict__ op, const double *__restrict__ field, double opd,
+                                         AdjState &q, const double *__restrict__ dk, double *sk) {
   const double *d = op->d;
-  const double *fx = field + __ldg(&op->i[4]);
-  const double *fy = fx + 121;
+  const double *fx = CF ? field + __ldg(&op->i[4]) : nullptr;
   const int nSlices = __ldg(&op->i[0]);
-  const double rho0 = __ldg(&d[BD_RHO0]);
-  const double opd = 1 + dp, opd2 = opd * opd;
-  const double r = opd * rsqrt_fast(fma(yp, yp, fma(xp, xp, 1.0)));
-  double X = x, QX = xp * r, Y = y, QY = yp * r;
-  double CX[TRK_ADJ_MAX_SLICES], CQX[TRK_ADJ_MAX_SLICES], CY[TRK_ADJ_MAX_SLICES], CQY[TRK_ADJ_MAX_SLICES];
-  for (int i = 0; i < nSlices; i++) {
-    CX[i] = X;
-    CQX[i] = QX;
-    CY[i] = Y;
-    CQY[i] = QY;
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-      cf_drift(d, j, rho0, opd2, X, QX, Y, QY);
-      if (j == 3)
-        break;
-      double Fx, Fy;
-      cf_fields(fx, fy, X, Y, Fx, Fy);
-      const double w = fma(__ldg(&d[BD_C2 + j]), X, __ldg(&d[BD_C1 + j]));
-      QX = fma(-w, Fy, QX);
-      QY = fma(w, Fx, QY);
+  const double rho0 = __ldg(&d[BD_RHO0]), iopd = rcp_fast(opd);
+  const double ka = __ldg(&d[BD_C2]) * iopd, kb = __ldg(&d[BD_C2 + 1]) * iopd;
+  adj_enter(q);
+  for (int i = nSlices; i >= 0; i--) {
+    /* the drift after slice i's last kick (slice 0: the entry drift), then the slice */
+    const bool end = i == nSlices || i == 0;
+    adj_rotate(q, rho0, __ldg(&d[end ? BD_SA : BD_SA2]), __ldg(&d[end ? BD_CA : BD_CA2]),
+               __ldg(&d[end ? BD_OMC : BD_OMC2]));
+    if (i == 0)
+      break;
+#pragma unroll 1
+    for (int j = 0; j < 3; j++) {
+      adj_bend_kick<CF>(q, j == 1 ? kb : ka, rho0, fx, dk, sk);
+      if (j < 2)
+        adj_rotate(q, rho0, __ldg(&d[BD_SA1]), __ldg(&d[BD_CA + 1]), __ldg(&d[BD_OMC + 1]));
     }
   }
-  /* exit: x = X, y = Y, (xp, yp) = (QX, QY) / sqrt(opd^2 - QX^2 - QY^2) */
-  double lX = lx, lY = ly, lQX = 0, lQY = 0, lopd = 0, sk1 = 0, sk2 = 0;
-  adj_m2s(QX, QY, opd, lxp, lyp, lQX, lQY, lopd);
-  for (int i = nSlices - 1; i >= 0; i--) {
-    /* substep entry states of slice i (and the kick positions) */
-    double sX[5], sQX[4], sY[5], sQY[4];
-    X = CX[i];
-    QX = CQX[i];
-    Y = CY[i];
-    QY = CQY[i];
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-      sX[j] = X;
-      sQX[j] = QX;
-      sY[j] = Y;
-      sQY[j] = QY;
-      cf_drift(d, j, rho0, opd2, X, QX, Y, QY);
-      sX[j + 1] = X;
-      sY[j + 1] = Y;
-      if (j == 3)
-        break;
-      double Fx, Fy;
-      cf_fields(fx, fy, X, Y, Fx, Fy);
-      const double w = fma(__ldg(&d[BD_C2 + j]), X, __ldg(&d[BD_C1 + j]));
-      QX = fma(-w, Fy, QX);
-      QY = fma(w, Fx, QY);
-    }
-#pragma unroll
-    for (int j = 3; j >= 0; j--) {
-      if (j < 3) {
-        /* kick at (X1, Y1) = (sX[j+1], sY[j+1]): QX -= w Fy, QY += w Fx */
-        const double X1 = sX[j + 1], Y1 = sY[j + 1];
-        const double c2 = __ldg(&d[BD_C2 + j]);
-        const double w = fma(c2, X1, __ldg(&d[BD_C1 + j]));
-        double Fx, Fy, Fyx, Fyy, Fxx, Fxy;
-        cf_fields(fx, fy, X1, Y1, Fx, Fy);
-        cf_fields_d(fx, fy, X1, Y1, Fyx, Fyy, Fxx, Fxy);
-        const double lw = fma(-lQX, Fy, lQY * Fx);
-        lX += lw * c2 + w * fma(-lQX, Fyx, lQY * Fxx);
-        lY += w * fma(-lQX, Fyy, lQY * Fxy);
-        if (dk) { /* d(kick)/dK1, d(kick)/dK2 with the adjoints after the kick */
-          double dFx, dFy;
-          cf_fields(dk, dk + 121, X1, Y1, dFx, dFy);
-          sk1 += w * (lQY * dFx - lQX * dFy);
-          cf_fields(dk + 242, dk + 363, X1, Y1, dFx, dFy);
-          sk2 += w * (lQY * dFx - lQX * dFy);
-        }
-      }
-      /* drift from (Xs, QXs, Ys, QYs): X' = Xs + u (omc fc + sa QXs),
-       * QX' = sa fc + ca QXs, Y' = Ys + QYs u sa, with
-       * fc = sqrt(opd^2 - QYs^2 - QXs^2), u = (rho0 + Xs) / (ca fc - sa QXs) */
-      const double Xs = sX[j], QXs = sQX[j], QYs = sQY[j];
-      const double sa = __ldg(&d[BD_SA + j]), ca = __ldg(&d[BD_CA + j]), omc = __ldg(&d[BD_OMC + j]);
-      const double fc = sqrt_nan(fma(-QXs, QXs, fma(-QYs, QYs, opd2)));
-      const double saq = sa * QXs;
-      const double fcosi = fma(ca, fc, -saq);
-      const double u = div_fast(rho0 + Xs, fcosi);
-      lQY += lY * u * sa;
-      const double lu = lY * QYs * sa + lX * fma(omc, fc, saq);
-      double lfc = lX * u * omc + lQX * sa;
-      double lsaq = lX * u;
-      double lQXs = lQX * ca;
-      double lXs = lX;
-      const double lfcosi = -lu * u / fcosi;
-      lXs += lu / fcosi;
-      lfc += ca * lfcosi;
-      lsaq -= lfcosi;
-      lQXs += sa * lsaq;
-      const double lu2 = lfc / (2 * fc);
-      lQXs -= 2 * QXs * lu2;
-      lopd += 2 * opd * lu2;
-      lQY -= 2 * QYs * lu2;
-      lX = lXs;
-      lQX = lQXs;
-    }
-  }
-  if (sk) {
-    sk[0] = sk1;
-    sk[1] = sk2;
-  }
-  /* entry: X = x, Y = y, (QX, QY) = opd (xp, yp) / sqrt(1 + xp^2 + yp^2) */
-  lx = lX;
-  ly = lY;
-  double lxp_in = 0, lyp_in = 0;
-  adj_s2m(xp, yp, opd, lQX, lQY, lxp_in, lyp_in, ldp);
-  lxp = lxp_in;
-  lyp = lyp_in;
-  ldp += lopd;
+  adj_leave(q);
 }
 
-/* forward pass from a checkpoint, recording every element's entry state */
-__global__ void adj_record_kernel(TrackArgs a, AdjArgs g) {
-  const long n = a.n, stride = (long)gridDim.x * blockDim.x;
-  for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
-    if (a.lost_pass[i] >= 0)
-      continue;
-    Part p;
-    p.x = g.ck[i];
-    p.xp = g.ck[n + i];
-    p.y = g.ck[2 * n + i];
-    p.yp = g.ck[3 * n + i];
-    p.s = 0;
-    p.dp = a.dp[i];
-    const trk_op *ops = a.ops;
-    if (a.ens_offsets)
-      ops += (long)ens_variant(a.ens_offsets, a.ens_variants, i) * a.ens_ops;
-    for (int k = 0; k < g.n_ops; k++) {
-      const trk_op *op = ops + k;
-      double *e = g.entry + (size_t)k * 4 * n;
-      e[i] = p.x;
-      e[n + i] = p.xp;
-      e[2 * n + i] = p.y;
-      e[3 * n + i] = p.yp;
-      switch (__ldg(&op->kind)) {
-      case OPK_DRIFT:
-        op_drift(op, p);
-        break;
-      case OPK_EDRIFT:
-      case OPK_RFDRIFT:
-        exact_drift(p, __ldg(&op->d[DD_L]));
-        break;
-      case OPK_MULT1:
-        op_mult1_fast(op, p, a.Po, 0.0, nullptr);
-        break;
-      case OPK_DIPOLE:
-        op_dipole_fast(op, p, a.Po, 0.0, nullptr);
-        break;
-      case OPK_CFBEND:
-        op_cfbend_fast(op, p, a.Po, 0.0, nullptr, a.field);
-        break;
-      default:
-        break;
-      }
-    }
-  }
-}
-
-/* one pass backwards: lambda at the end of the pass -> at its start */
-__global__ void __launch_bounds__(128) adj_reverse_kernel(TrackArgs a, AdjArgs g) {
+/* every pass of the run backwards, one particle per thread */
+__global__ void __launch_bounds__(128, 4) adj_reverse_kernel(TrackArgs a, AdjArgs g) {
   const long n = a.n;
   const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
   const bool act = i < n && a.lost_pass[i] < 0;
-  double lx = 0, lxp = 0, ly = 0, lyp = 0, ldp = 0, dp = 0;
   /* variant of this particle (ensembles); lanes past the end take the last
    * particle's, so a warp of one variant stays uniform */
   int v = 0;
@@ -3880,75 +3681,80 @@ __global__ void __launch_bounds__(128) adj_reverse_kernel(TrackArgs a, AdjArgs g
     v = ens_variant(a.ens_offsets, a.ens_variants, i < n ? i : n - 1);
   const trk_op *ops = a.ops + (long)v * a.ens_ops;
   const bool warp_uniform = __all_sync(0xffffffffu, v == __shfl_sync(0xffffffffu, v, 0));
+  /* idle lanes carry a particle at rest on the axis */
+  AdjState q = {0, 0, 0, 0, 0, 0, 0, 0};
+  double opd = 1;
   if (act) {
-    lx = g.lam[i];
-    lxp = g.lam[n + i];
-    ly = g.lam[2 * n + i];
-    lyp = g.lam[3 * n + i];
-    ldp = g.lam[4 * n + i];
-    dp = a.dp[i];
+    q.x = a.x[i];
+    q.px = a.xp[i];
+    q.y = a.y[i];
+    q.py = a.yp[i];
+    opd = 1 + a.dp[i];
+    /* dL/dx = (2 x + 2 w mean(x))/N over the variant's survivors, same in y */
+    const double *c = g.coef + 3 * v;
+    q.lx = fma(2 * q.x, c[2], c[0]);
+    q.ly = fma(2 * q.y, c[2], c[1]);
   }
-  for (int k = g.n_ops - 1; k >= 0; k--) {
-    const trk_op *op = ops + k;
-    double x = 0, xp = 0, y = 0, yp = 0;
-    if (act) {
-      const double *e = g.entry + (size_t)k * 4 * n;
-      x = e[i];
-      xp = e[n + i];
-      y = e[2 * n + i];
-      yp = e[3 * n + i];
+  for (long t = g.n_passes - 1; t >= 0; t--) {
+    if (act && t < g.n_passes - 1) {
+      const double *e = g.ck + (size_t)t * 4 * n;
+      q.x = e[i];
+      q.px = e[n + i];
+      q.y = e[2 * n + i];
+      q.py = e[3 * n + i];
     }
-    double sens = 0, sk[2] = {0, 0};
-    const int prm = __ldg(&g.op_param[k]);
-    const int dfo = g.op_dfield ? __ldg(&g.op_dfield[k]) : -1;
-    const double *dk = (prm >= 0 && dfo >= 0) ? g.dfield + dfo : nullptr;
-    bool two = false;
-    switch (__ldg(&op->kind)) {
-    case OPK_DRIFT:
-    case OPK_EDRIFT:
-    case OPK_RFDRIFT: {
-      const double L = __ldg(&op->d[DD_L]);
-      lxp += L * lx;
-      lyp += L * ly;
-      break;
-    }
-    case OPK_MULT1:
-      sens = adj_mult1(op, g.op_dk + 3 * ((long)v * g.n_ops + k), x, xp, y, yp, dp, lx, lxp, ly, lyp, ldp);
-      break;
-    case OPK_DIPOLE:
-      adj_dipole(op, x, xp, y, yp, dp, lx, lxp, ly, lyp, ldp, dk, sk);
-      two = dk != nullptr;
-      break;
-    case OPK_CFBEND:
-      adj_cfbend(op, a.field, x, xp, y, yp, dp, lx, lxp, ly, lyp, ldp, dk, sk);
-      two = dk != nullptr;
-      break;
-    default:
-      break;
-    }
-    if (prm >= 0) {
-      /* one parameter (multipole K) or two (CSBEND K1, K2 at prm, prm + 1) */
-      for (int q = 0; q < (two ? 2 : 1); q++) {
-        double sv = two ? sk[q] : sens;
-        if (!act)
-          sv = 0;
-        if (warp_uniform) {
-          for (int off = 16; off > 0; off >>= 1)
-            sv += __shfl_xor_sync(0xffffffffu, sv, off);
-          if ((threadIdx.x & 31) == 0 && sv != 0)
-            atomicAdd(&g.grad[(long)v * g.n_params + prm + q], sv);
-        } else if (sv != 0) {
-          atomicAdd(&g.grad[(long)v * g.n_params + prm + q], sv);
+    for (int k = g.n_ops - 1; k >= 0; k--) {
+      const trk_op *op = ops + k;
+      double sk[2] = {0, 0};
+      const int prm = __ldg(&g.op_param[k]);
+      const int dfo = __ldg(&g.op_dfield[k]);
+      const double *dk = (prm >= 0 && dfo >= 0) ? g.dfield + dfo : nullptr;
+      switch (__ldg(&op->kind)) {
+      case OPK_DRIFT:
+      case OPK_EDRIFT:
+      case OPK_RFDRIFT: {
+        const double L = __ldg(&op->d[DD_L]);
+        q.x = fma(-L, q.px, q.x);
+        q.y = fma(-L, q.py, q.y);
+        q.lpx = fma(L, q.lx, q.lpx);
+        q.lpy = fma(L, q.ly, q.lpy);
+        break;
+      }
+      case OPK_MULT1: {
+        const double *mk = g.op_dk + 3 * ((long)v * g.n_ops + k);
+        const int order = __ldg(&op->i[4]) & 0xff;
+        if (order == 1)
+          sk[0] = adj_mult1<1>(op, mk, opd, q);
+        else if (order == 2)
+          sk[0] = adj_mult1<2>(op, mk, opd, q);
+        else
+          sk[0] = adj_mult1<3>(op, mk, opd, q);
+        break;
+      }
+      case OPK_DIPOLE:
+        adj_bend<false>(op, a.field, opd, q, dk, sk);
+        break;
+      case OPK_CFBEND:
+        adj_bend<true>(op, a.field, opd, q, dk, sk);
+        break;
+      default:
+        break;
+      }
+      if (prm >= 0) {
+        /* one parameter (multipole K) or two (CSBEND K1, K2 at prm, prm + 1) */
+        for (int m = 0; m < (dk ? 2 : 1); m++) {
+          double sv = act ? sk[m] : 0;
+          if (warp_uniform) {
+            for (int off = 16; off > 0; off >>= 1)
+              sv += __shfl_xor_sync(0xffffffffu, sv, off);
+            if ((threadIdx.x & 31) == 0 && sv != 0)
+              atomicAdd(&g.grad[(long)v * g.n_params + prm + m], sv);
+          } else if (sv != 0) {
+            atomicAdd(&g.grad[(long)v * g.n_params + prm + m], sv);
+          }
         }
       }
     }
-  }
-  if (act) {
-    g.lam[i] = lx;
-    g.lam[n + i] = lxp;
-    g.lam[2 * n + i] = ly;
-    g.lam[3 * n + i] = lyp;
-    g.lam[4 * n + i] = ldp;
   }
 }
 #endif
@@ -4083,17 +3889,6 @@ void launch_track_ensemble(const TrackArgs &a, const long *offsets, int n_varian
   e.ens_variants = n_variants;
   e.ens_ops = ops_per_variant;
   launch_track(e, ensemble_variant_ok(variant) ? variant : 1, lean, n, max_blocks, st);
-}
-
-void launch_adjoint_record(const TrackArgs &a, const AdjArgs &g, cudaStream_t st) {
-#if TRK_FAST
-  const long grid = std::min<long>((a.n + 127) / 128, 148L * 64);
-  adj_record_kernel<<<(int)std::max<long>(grid, 1), 128, 0, st>>>(a, g);
-#else
-  (void)a;
-  (void)g;
-  (void)st;
-#endif
 }
 
 void launch_adjoint_reverse(const TrackArgs &a, const AdjArgs &g, cudaStream_t st) {

@@ -112,19 +112,20 @@ struct WakeArgs {
 };
 
 /* reverse-mode adjoint of the fast build's element maps (DRIF, EDRIFT,
- * single-order multipoles, pure-dipole CSBEND) */
+ * single-order multipoles, CSBEND pure dipoles and K1/K2 expansions) */
 struct AdjArgs {
-  const double *ck;      /* checkpoint of the pass being reversed: x, xp, y, yp columns of n */
-  double *entry;         /* element entry states: [op][4][n] */
-  double *lam;           /* adjoint of x, xp, y, yp, delta: 5 columns of n */
+  const double *ck;      /* beam at the end of pass t (t < n_passes - 1) at ck + t * 4 n: x, xp, y, yp columns */
+  const double *coef;    /* per variant: loss gradient coefficients (2 w mean(x)/N, 2 w mean(y)/N, 1/N) */
   double *grad;          /* gradient accumulators, one per parameter */
   const int *op_param;   /* parameter index of each op, -1 if none */
   const double *op_dk;   /* per variant and op: d(kick strength)/d(parameter) of kick steps 0..2 */
   const int *op_dfield;  /* per op: offset in dfield of a CSBEND's field derivatives (-1 none) */
-  const double *dfield;  /* d(Fx, Fy)/dK1 and d(Fx, Fy)/dK2 tables, 4 x 121 doubles per CSBEND op */
+  const double *dfield;  /* d(Fx, Fy)/dK1 then /dK2, TRK_DFIELD_LEN doubles per distinct CSBEND, packed (adj_dfield) */
+  long n_passes;
   int n_ops;             /* ops per variant */
   int n_params;          /* parameters per variant (grad holds n_variants x n_params) */
 };
+#define TRK_DFIELD_LEN 16
 
 #define TRK_DECLARE_LAUNCHERS(NS)                                                                            \
   namespace NS {                                                                                             \
@@ -143,7 +144,6 @@ struct AdjArgs {
                     int elem, int grid, cudaStream_t st);                                                    \
   void launch_matrix(const TrackArgs &a, const double *m, int order, int grid, cudaStream_t st);             \
   int ensemble_variant_ok(int variant);                                                                      \
-  void launch_adjoint_record(const TrackArgs &a, const AdjArgs &g, cudaStream_t st);                         \
   void launch_adjoint_reverse(const TrackArgs &a, const AdjArgs &g, cudaStream_t st);                        \
   void launch_track_ensemble(const TrackArgs &a, const long *offsets, int n_variants, int ops_per_variant,   \
                              int variant, int lean, long n, int max_blocks, cudaStream_t st);               \

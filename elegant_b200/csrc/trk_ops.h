@@ -62,7 +62,7 @@ enum trk_op_kind {
 #define BF_RADE1 128   /* SYNCH_RAD with an entrance edge angle: delta pre-adjusted at the entrance */
 #define BF_RADE2 256   /* ... and post-adjusted at the exit */
 #define BF_MERGED 512  /* substep angles small enough for the fast build's merged body */
-#define BF_LINEAR 1024 /* combined function: midplane field linear in x (no K2 or higher terms) */
+#define BF_LINEAR 1024 /* combined function: midplane field linear in x, its slope constant (K1 only) */
 
 /* RF flags (i[3]) */
 #define RF_SAME_DGAMMA 1
