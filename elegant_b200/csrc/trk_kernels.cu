@@ -667,6 +667,75 @@ done:
 
 /* ---------------------------------------------------------------- CSBEND */
 #if !TRK_FAST
+/* Drift substep of a pure-dipole CSBEND in the parity build, every operation
+ * rounded as the reference rounds it (src/csbend.c:1580-1606), and the loss
+ * conditions before any coordinate of the substep changes: |QX/f| > 1 and
+ * cos(dsh/rho0 + phi) == 0. */
+struct DipoleDrift {
+  double X, QX, Y, dist;
+  int ok;
+};
+
+__device__ __noinline__ DipoleDrift dipole_drift_checked(double arg, double rho0, double f, double yf, double opd,
+                                                         double X, double QX, double Y, double QY, double dist) {
+  DipoleDrift r = {X, QX, Y, dist, 0};
+  const double sin_phi = trkcr_div_rcp(QX, f, yf);
+  if (fabs(sin_phi) > 1)
+    return r;
+  const double phi = trkcr_asin(sin_phi);
+  double sine, cosi;
+  trkcr_sincos(__dadd_rn(arg, phi), &sine, &cosi);
+  if (cosi == 0)
+    return r;
+  const double tang = __ddiv_rn(sine, cosi);
+  const double cos_phi = trkcr_cos(phi);
+  r.QX = __dmul_rn(f, sine);
+  const double a3 = trkcr_div_rcp(__dmul_rn(__dadd_rn(rho0, X), cos_phi), f, yf);
+  const double factor = __dmul_rn(a3, __dsub_rn(tang, __ddiv_rn(sin_phi, cos_phi)));
+  r.Y = __dadd_rn(Y, __dmul_rn(QY, factor));
+  r.dist = __dadd_rn(dist, __dmul_rn(factor, opd));
+  const double fr = __ddiv_rn(cos_phi, cosi);
+  r.X = __dadd_rn(__dmul_rn(rho0, __dsub_rn(fr, 1.0)), __dmul_rn(fr, X));
+  r.ok = 1;
+  return r;
+}
+
+/* a / b rounded as IEEE rounds it, from yh = RN(1/b) and yl = RN(1/b - yh):
+ * q0 = RN(a yh + RN(a yl)) is faithful (within 1/2 + 2^-50 ulp), so one
+ * correction gives RN(a/b) by Markstein's theorem (trkcr_div_rcp).  No range
+ * checks: the caller keeps a and the quotient normal. */
+__device__ __forceinline__ double div_hl(double a, double b, double yh, double yl) {
+  const double q0 = __fma_rn(a, yh, __dmul_rn(a, yl));
+  return __fma_rn(__fma_rn(-b, q0, a), yh, q0);
+}
+
+/* the same from yh alone: two corrections (trkcr_div_rcp without its checks) */
+__device__ __forceinline__ double div_h(double a, double b, double yh) {
+  const double q0 = __dmul_rn(a, yh);
+  const double q1 = __fma_rn(__fma_rn(-b, q0, a), yh, q0);
+  return __fma_rn(__fma_rn(-b, q1, a), yh, q1);
+}
+
+/* RN(1/b) for 1 - 2^-15 <= b <= 1: with d = 1 - b exact, 1 + d + d^2 + d^3 is
+ * faithful (d^4 is under 2^-7 of half an ulp), and one Newton step from a
+ * faithful value rounds correctly unless b's significand is all ones
+ * (Markstein), b = 1 - 2^-53, which the caller excludes. */
+__device__ __forceinline__ double rcp_below1(double b) {
+  const double d = __dsub_rn(1.0, b);
+  const double y0 = __fma_rn(d, __fma_rn(d, __dadd_rn(1.0, d), 1.0), 1.0);
+  return __fma_rn(y0, __fma_rn(-b, y0, 1.0), y0);
+}
+
+/* lead + c with the rounding test of trkcr_tiny_test; the bits in which the
+ * two bounds' sums differ are added to *bad instead of branching */
+__device__ __forceinline__ double tiny_sum(double lead, double c, unsigned long long *bad) {
+  const double ac = fabs(c);
+  const double u = __dadd_rn(lead, __fma_rn(ac, 0x1p-49, c));
+  const double v = __dadd_rn(lead, __fma_rn(-ac, 0x1p-49, c));
+  *bad |= (unsigned long long)(__double_as_longlong(u) ^ __double_as_longlong(v));
+  return u;
+}
+
 /* Body of a pure-dipole CSBEND in the parity build: integrate_csbend_ordn
  * (src/csbend.c:1561-1660) with Fx = 0, Fy = 1 and no radiation, every
  * operation rounded as the reference rounds it, with these shortcuts that
@@ -674,73 +743,126 @@ done:
  *  - 1 + delta is constant through the body, and so is f = sqrt((1+delta)^2
  *    - QY^2) while QY^2 rounds to the same double (QY moves only by the
  *    (1+delta) divide/multiply round trip, by an ulp at most): f and its
- *    reciprocal are re-formed only when QY^2 changes;
- *  - divisions by f, rho0, rho_actual and 1 + delta use their correctly
- *    rounded reciprocals, formed once (trkcr_div_rcp: Markstein's two FMA
- *    corrections give the IEEE quotient for five FP64 operations, about a
- *    third of an IEEE division's cost on B200);
- *  - the kick's Fx term, ((ds (1 + X/rho0)) 0)/rho_actual, is a signed zero
- *    (or NaN), formed by multiplying by 1/rho_actual instead of dividing;
+ *    reciprocal are re-formed only when QY^2 changes.  Once a round trip
+ *    returns the QY it was given, every later one does, and QY is left alone;
+ *  - a substep runs straight through without a branch: the tiny-argument
+ *    forms of asin, sin and cos (trk_crmath.h: |x| <= 2^-7; below 2^-26 their
+ *    corrections vanish in the rounding, as they must) with the outcome of
+ *    their rounding tests collected in one word, quotients by Markstein's
+ *    corrections (by f, rho0, rho_actual, 1 + delta from double-double
+ *    reciprocals formed once, by the two cosines from rcp_below1), and the
+ *    range that all of this needs in two integer maxima.  If anything fails,
+ *    the substep is redone by dipole_drift_checked, for one warp in 70 on the
+ *    FODO ring's bends;
+ *  - the kick's Fx term, ((ds (1 + X/rho0)) 0)/rho_actual, is a signed zero;
  *  - dz_lost is summed only for a lost particle, from the substeps done.
  * Loss conditions, their order and the state left at a loss are the
- * reference's: aperture at the start of each slice, f <= 0, |QX/f| > 1 and
- * cos(dsh/rho0 + phi) == 0 before any coordinate of the substep changes. */
+ * reference's: aperture at the start of each slice, f <= 0, then those of
+ * dipole_drift_checked.
+ * Bound by FP64 issue (56 % of the pipe) and the chain of the three functions;
+ * a substep takes 114 FP64 operations of 225 instructions, where the branching
+ * form, with IEEE divisions and a test after every function, took 170 of 390.
+ * With op_mult1_exact, FODO ring with RF and wake, 1e6 particles: 92.7 -> 57.7
+ * ms per turn; 30,011 particles through the ring with sextupoles: 7.7 -> 3.8. */
+#define TRK_TINY_HI 0x3f7fff00u  /* high word just below 2^-7 */
+#define TRK_NORMAL_HI 0x07b00000u /* of 2^-900: quotients and residuals stay normal above */
+#define TRK_X_HI 0x40900000u     /* of 2^10 */
 __device__ __forceinline__ bool bend_dipole_exact(const double *__restrict__ d, int nSlices, int nSub, double rho0,
                                                   bool roundtrip, const trk_aperture *ap, bool aptilt, double apc,
                                                   double aps, double &X, double &QX, double &Y, double &QY,
                                                   const double D, double &dist, int &done) {
   const double opd = __dadd_rn(1.0, D);
   const double opd2 = __dmul_rn(opd, opd);
-  const double yopd = __drcp_rn(opd);
-  const double yrho0 = __ldg(&d[BD_RHOINV]);
+  const double yopd = __drcp_rn(opd), yopdl = __dmul_rn(__fma_rn(-opd, yopd, 1.0), yopd);
+  const double yrho0 = __ldg(&d[BD_RHOINV]), yrho0l = __dmul_rn(__fma_rn(-rho0, yrho0, 1.0), yrho0);
   const double rho_a = __ldg(&d[BD_RHOA]), yrho_a = __ldg(&d[BD_INVRHOA]);
+  const double yrho_al = __dmul_rn(__fma_rn(-rho_a, yrho_a, 1.0), yrho_a);
   double qy2 = __dmul_rn(QY, QY);
   double f2 = __dsub_rn(opd2, qy2);
   double f = __dsqrt_rn(f2);
-  double yf = __drcp_rn(f);
+  double yf = __drcp_rn(f), yfl = __dmul_rn(__fma_rn(-f, yf, 1.0), yf);
+  /* the straight path wants ordinary divisors: 2^-10 <= f, 1 + delta, |rho| < 2^20 */
+  const unsigned hf = (unsigned)__double2hiint(f), ho = (unsigned)__double2hiint(opd), hr = hi_abs(rho0),
+                 ha = hi_abs(rho_a);
+  const bool plain = min(min(hf, ho), min(hr, ha)) >= 0x3f500000u && max(max(hf, ho), max(hr, ha)) < 0x41300000u;
+  bool qy_moves = true;
   done = 0;
   for (int i = 0; i < nSlices; i++) {
     if (!check_aperture(X, Y, ap, aptilt, apc, aps))
       return false;
+#pragma unroll 1
     for (int j = 0; j < nSub; j++) {
       if (f2 <= 0)
         return false;
-      const double sin_phi = trkcr_div_rcp(QX, f, yf);
-      if (fabs(sin_phi) > 1)
-        return false;
-      const double phi = trkcr_asin(sin_phi);
-      double sine, cosi;
-      trkcr_sincos(__dadd_rn(__ldg(&d[BD_ARG + j]), phi), &sine, &cosi);
-      if (cosi == 0)
-        return false;
-      const double tang = __ddiv_rn(sine, cosi);
-      const double cos_phi = trkcr_cos(phi);
-      QX = __dmul_rn(f, sine);
-      const double a3 = trkcr_div_rcp(__dmul_rn(__dadd_rn(rho0, X), cos_phi), f, yf);
-      const double factor = __dmul_rn(a3, __dsub_rn(tang, __ddiv_rn(sin_phi, cos_phi)));
-      Y = __dadd_rn(Y, __dmul_rn(QY, factor));
-      dist = __dadd_rn(dist, __dmul_rn(factor, opd));
+      const double arg = __ldg(&d[BD_ARG + j]);
+      unsigned long long bad = 0;
+      const double sin_phi = div_hl(QX, f, yf, yfl);
+      double z = __dmul_rn(sin_phi, sin_phi);
+      const double phi = tiny_sum(sin_phi, trkcr_asin_tiny_c(sin_phi, z), &bad);
+      const double t = __dadd_rn(arg, phi);
+      z = __dmul_rn(t, t);
+      const double sine = tiny_sum(t, trkcr_sin_tiny_c(t, z), &bad);
+      const double cosi = tiny_sum(1.0, trkcr_cos_tiny_c(z), &bad);
+      const double cos_phi = tiny_sum(1.0, trkcr_cos_tiny_c(__dmul_rn(phi, phi)), &bad);
+      const double yi = rcp_below1(cosi);
+      const double tang = div_h(sine, cosi, yi), fr = div_h(cos_phi, cosi, yi);
+      const double tphi = div_h(sin_phi, cos_phi, rcp_below1(cos_phi));
+      const double a3 = div_hl(__dmul_rn(__dadd_rn(rho0, X), cos_phi), f, yf, yfl);
+      const double factor = __dmul_rn(a3, __dsub_rn(tang, tphi));
+      const unsigned tiny = max(hi_abs(sin_phi), hi_abs(t)), least = min(hi_abs(QX), hi_abs(t));
+      const unsigned long long ones = 0x3fefffffffffffffULL; /* 1 - 2^-53 */
+      const bool fine = plain && bad == 0 && tiny < TRK_TINY_HI && least >= TRK_NORMAL_HI && hi_abs(X) < TRK_X_HI &&
+                        (unsigned long long)__double_as_longlong(cosi) != ones &&
+                        (unsigned long long)__double_as_longlong(cos_phi) != ones;
+      if (fine) {
+        QX = __dmul_rn(f, sine);
+        Y = __dadd_rn(Y, __dmul_rn(QY, factor));
+        dist = __dadd_rn(dist, __dmul_rn(factor, opd));
+        X = __dadd_rn(__dmul_rn(rho0, __dsub_rn(fr, 1.0)), __dmul_rn(fr, X));
+      } else {
+        const DipoleDrift r = dipole_drift_checked(arg, rho0, f, yf, opd, X, QX, Y, QY, dist);
+        if (!r.ok)
+          return false;
+        X = r.X;
+        QX = r.QX;
+        Y = r.Y;
+        dist = r.dist;
+      }
       done++;
-      const double fr = __ddiv_rn(cos_phi, cosi);
-      X = __dadd_rn(__dmul_rn(rho0, __dsub_rn(fr, 1.0)), __dmul_rn(fr, X));
       if (j == nSub - 1)
         break;
       /* kick: QX += -ds (1 + X/rho0) Fy / rho_a, QY += ds (1 + X/rho0) Fx / rho_a */
       const double ds = __ldg(&d[BD_DS + j]);
-      const double w = __dmul_rn(ds, __dadd_rn(1.0, trkcr_div_rcp(X, rho0, yrho0)));
-      QX = __dadd_rn(QX, trkcr_div_rcp(-w, rho_a, yrho_a));
-      QY = __dadd_rn(QY, __dmul_rn(__dmul_rn(w, 0.0), yrho_a));
-      if (roundtrip) {
-        /* QX /= (1 + delta); QY /= ...; QX *= (1 + delta); QY *= ... */
-        QX = __dmul_rn(trkcr_div_rcp(QX, opd, yopd), opd);
-        QY = __dmul_rn(trkcr_div_rcp(QY, opd, yopd), opd);
+      const bool pk = plain && hi_abs(X) - TRK_NORMAL_HI < TRK_X_HI - TRK_NORMAL_HI;
+      double w;
+      if (pk) {
+        w = __dmul_rn(ds, __dadd_rn(1.0, div_hl(X, rho0, yrho0, yrho0l)));
+        QX = __dadd_rn(QX, div_hl(-w, rho_a, yrho_a, yrho_al));
+      } else {
+        w = __dmul_rn(ds, __dadd_rn(1.0, trkcr_div_rcp(X, rho0, yrho0)));
+        QX = __dadd_rn(QX, trkcr_div_rcp(-w, rho_a, yrho_a));
       }
-      const double q2 = __dmul_rn(QY, QY);
-      if (q2 != qy2) {
-        qy2 = q2;
-        f2 = __dsub_rn(opd2, qy2);
-        f = __dsqrt_rn(f2);
-        yf = __drcp_rn(f);
+      if (roundtrip) {
+        /* QX /= (1 + delta); QX *= (1 + delta) */
+        if (pk && hi_abs(QX) - TRK_NORMAL_HI < TRK_X_HI - TRK_NORMAL_HI)
+          QX = __dmul_rn(div_hl(QX, opd, yopd, yopdl), opd);
+        else
+          QX = __dmul_rn(trkcr_div_rcp(QX, opd, yopd), opd);
+      }
+      if (qy_moves || !pk) {
+        const double before = QY;
+        QY = __dadd_rn(QY, __dmul_rn(__dmul_rn(w, 0.0), yrho_a));
+        if (roundtrip)
+          QY = __dmul_rn(trkcr_div_rcp(QY, opd, yopd), opd);
+        qy_moves = !(pk && QY == before && QY != 0);
+        const double q2 = __dmul_rn(QY, QY);
+        if (q2 != qy2) {
+          qy2 = q2;
+          f2 = __dsub_rn(opd2, qy2);
+          f = __dsqrt_rn(f2);
+          yf = __drcp_rn(f);
+          yfl = __dmul_rn(__fma_rn(-f, yf, 1.0), yf);
+        }
       }
     }
   }
@@ -1711,6 +1833,122 @@ __device__ __forceinline__ bool op_bend(const trk_op *__restrict__ op, Part &p, 
 }
 
 #if !TRK_FAST
+/* op_mult restricted to OPK_MULT1 (one normal multipole, 4th-order integrator
+ * with drifts, no misalignment, steering, radiation or fringe), with the same
+ * roundings:
+ *  - the first conversion to slopes after a kick is used for its loss test
+ *    only, the one after the (1 + delta) round trip gives the slopes; the two
+ *    share the root and its reciprocal while their radicands are equal, which
+ *    the ulp the trip can move a momentum by hardly ever changes;
+ *  - quotients by 1 + delta and by the roots through their correctly rounded
+ *    reciprocals (trkcr_div_rcp);
+ *  - the conversion after the last drift repeats the last kick's;
+ *  - dzLoss is summed only for a lost particle.
+ * One copy of the substep, not unrolled: the general body's unrolled divisions
+ * and roots ran out of the instruction cache in every element. */
+__device__ __forceinline__ bool op_mult1_exact(const trk_op *__restrict__ op, Part &p, double Po, double z_start,
+                                               const trk_aperture *ap) {
+  const int n_parts = __ldg(&op->i[0]);
+  const int order = __ldg(&op->i[4]) & 0xff;
+  const int flags = __ldg(&op->i[6]);
+  const double *d = op->d;
+  const bool aptilt = (flags & MF_APTILT) != 0;
+  const double apc = __ldg(&d[MD_APC]), aps = __ldg(&d[MD_APS]);
+  double x = p.x, xp = p.xp, y = p.y, yp = p.yp, s = 0;
+  const double opd = 1 + p.dp, opd2 = opd * opd, yopd = __drcp_rn(opd);
+  bool ok = true;
+  int done = 0;
+  if (!(max(hi_abs(x), hi_abs(y)) < 0x40240000u && max(hi_abs(xp), hi_abs(yp)) < 0x3ff00000u) &&
+      (isnan(x) || isnan(xp) || isnan(y) || isnan(yp) || fabs(x) > TRK_COORD_LIMIT || fabs(y) > TRK_COORD_LIMIT ||
+       fabs(xp) > TRK_SLOPE_LIMIT || fabs(yp) > TRK_SLOPE_LIMIT)) {
+    p.s = z_start + __ldg(&d[MD_DZFULL]); /* as in op_mult */
+    p.dp = Po * (1 + p.dp);
+    return false;
+  }
+  double root = sqrt(1 + sqr(xp) + sqr(yp)), yroot = __drcp_rn(root);
+  double qx = trkcr_div_rcp(opd * xp, root, yroot), qy = trkcr_div_rcp(opd * yp, root, yroot);
+  double rad = opd2 - qx * qx - qy * qy;
+  if (rad <= 0)
+    ok = false;
+  else {
+    root = sqrt(rad);
+    yroot = __drcp_rn(root);
+    xp = trkcr_div_rcp(qx, root, yroot);
+    yp = trkcr_div_rcp(qy, root, yroot);
+  }
+#pragma unroll 1
+  for (int k = 0; ok && k < 4 * n_parts; k++) {
+    const int step = k & 3;
+    if (step == 0 && !check_aperture(x, y, ap, aptilt, apc, aps)) {
+      p.x = x;
+      p.y = y;
+      ok = false;
+      break;
+    }
+    const double dsh = __ldg(&d[MD_DSH + step]);
+    x += xp * dsh;
+    y += yp * dsh;
+    s += dsh * sqrt(1 + sqr(xp) + sqr(yp));
+    done++;
+    if (step == 3)
+      continue; /* kickFrac of the last substep is 0 */
+    if (flags & MF_KNL0) {
+      const double K = __ldg(&d[MD_KQ + step * 3]);
+      double sFx, sFy;
+      if (order == 1) {
+        sFy = x;
+        sFx = y;
+      } else if (order == 2) {
+        const double x2 = x * x, y2 = y * y;
+        sFy = 0.5 * x2 + (-0.5) * y2;
+        sFx = x * y;
+      } else {
+        const double x2 = x * x, y2 = y * y;
+        const double x3 = x2 * x, y3 = y2 * y;
+        sFy = c_coef[6] * x3 + (c_coef[8] * x) * y2;
+        sFx = (c_coef[7] * x2) * y + c_coef[9] * y3;
+      }
+      qx -= K * sFy;
+      qy += K * sFx;
+    }
+    const double rad1 = opd2 - qx * qx - qy * qy;
+    qx = trkcr_div_rcp(qx, opd, yopd) * opd;
+    qy = trkcr_div_rcp(qy, opd, yopd) * opd;
+    rad = opd2 - qx * qx - qy * qy;
+    if (rad1 <= 0 || rad <= 0) {
+      ok = false;
+      break;
+    }
+    root = sqrt(rad);
+    yroot = __drcp_rn(root);
+    xp = trkcr_div_rcp(qx, root, yroot);
+    yp = trkcr_div_rcp(qy, root, yroot);
+  }
+  if (ok && !check_aperture(x, y, ap, aptilt, apc, aps)) {
+    p.x = x;
+    p.y = y;
+    ok = false;
+  }
+  if (ok) {
+    p.x = x;
+    p.xp = xp;
+    p.y = y;
+    p.yp = yp;
+    p.s += s;
+    ok = (max(hi_abs(x), hi_abs(y)) < 0x40240000u && max(hi_abs(xp), hi_abs(yp)) < 0x3ff00000u) ||
+         !(isnan(x) || isnan(xp) || isnan(y) || isnan(yp) || fabs(x) > TRK_COORD_LIMIT || fabs(y) > TRK_COORD_LIMIT ||
+           fabs(xp) > TRK_SLOPE_LIMIT || fabs(yp) > TRK_SLOPE_LIMIT);
+  }
+  if (!ok) {
+    double dzLoss = 0;
+    for (int k = 0; k < done; k++)
+      dzLoss += __ldg(&d[MD_DSH + (k & 3)]);
+    p.s = z_start + dzLoss;
+    p.dp = Po * (1 + p.dp);
+  }
+  return ok;
+}
+
 /* op_bend restricted to what a plain pure dipole reaches (OPK_DIPOLE: no
  * misalignment, tilt, radiation, field expansion or expanded Hamiltonian;
  * edges at most the linear kick), with the same operations in the same
@@ -2810,7 +3048,7 @@ __device__ __forceinline__ bool track_particle(const TrackArgs &a, const trk_op 
 #if TRK_FAST
         ok = op_mult1(op, p, a.Po, h.z_start, ap_in);
 #else
-        ok = op_mult(op, p, a.Po, h.z_start, ap_in);
+        ok = op_mult1_exact(op, p, a.Po, h.z_start, ap_in);
 #endif
         break;
       case OPK_DIPOLE:
