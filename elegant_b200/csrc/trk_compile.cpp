@@ -1030,16 +1030,20 @@ int trk_compile(const trk_lattice *l, double Po, CompiledLattice &out) {
       const int f = op.i[6];
       const int o = op.i[4] & 0xff;
       if (op.i[1] == 4 && !op.i[2] && op.d[MD_DRIFT] != 0 && o >= 1 && o <= 3 && !(op.i[5] & 1) &&
-          !(f & (MF_KNL1 | MF_KNL2 | MF_XKICK | MF_YKICK | MF_OFFSET | MF_TILT | MF_ENDDRIFT | MF_RAD | MF_FRINGE1 |
-                 MF_FRINGE2)))
-        op.kind = OPK_MULT1;
+          !(f & (MF_KNL1 | MF_KNL2 | MF_XKICK | MF_YKICK | MF_OFFSET | MF_TILT | MF_ENDDRIFT | MF_FRINGE1 |
+                 MF_FRINGE2))) {
+        if (f & MF_RAD)
+          op.i[6] |= MF_MERGED;
+        else
+          op.kind = OPK_MULT1;
+      }
     } else if (op.kind == OPK_BEND) {
       const bool e1_noop = op.i[5] == EDGE_NONE ||
                            (op.i[5] == EDGE_LIN1 && op.d[BD_TE1] == 0 && op.d[BD_PSI1] == 0 && op.d[BD_LIM1] <= 0);
       const bool e2_noop = op.i[6] == EDGE_NONE ||
                            (op.i[6] == EDGE_LIN1 && op.d[BD_TE2] == 0 && op.d[BD_PSI2] == 0 && op.d[BD_LIM2] <= 0);
-      const bool plain =
-        op.i[1] == 4 && !(op.i[7] & (BF_MISALIGN | BF_APTILT | BF_RAD | BF_EXPAND)) && e1_noop && e2_noop;
+      const bool but_rad = op.i[1] == 4 && !(op.i[7] & (BF_MISALIGN | BF_APTILT | BF_EXPAND)) && e1_noop && e2_noop;
+      const bool plain = but_rad && !(op.i[7] & BF_RAD);
       if (plain && op.i[2] == 0)
         op.kind = OPK_DIPOLE;
       else if (plain && op.i[2] == 1 && op.i[3] == 5) {
@@ -1055,7 +1059,9 @@ int trk_compile(const trk_lattice *l, double Po, CompiledLattice &out) {
        * integrator's overshoot after the second kick); below 0.010 a particle
        * keeps more than 5e-3 for its own slope.  Bends of larger slice angles
        * go to the checked bodies at once rather than through both. */
-      if (plain && 0.8512 * std::fabs(op.d[BD_SLICE] / op.d[BD_RHO0]) < 0.010)
+      const bool body = op.kind == OPK_DIPOLE || op.kind == OPK_CFBEND ||
+                        (but_rad && (op.i[7] & BF_RAD) && op.i[2] == 0 && !(op.i[7] & (BF_RADE1 | BF_RADE2)));
+      if (body && 0.8512 * std::fabs(op.d[BD_SLICE] / op.d[BD_RHO0]) < 0.010)
         op.i[7] |= BF_MERGED;
     }
     if (op.kind != OPK_NOP && op.kind != OPK_DRIFT && op.kind != OPK_EDRIFT && op.kind != OPK_RFDRIFT &&

@@ -2812,6 +2812,225 @@ __device__ __forceinline__ bool op_cfbend(const trk_op *__restrict__ op, Part &p
   p = r.p;
   return !r.lost;
 }
+/* ------------------------------------ the same with synchrotron radiation
+ * The reference takes the energy loss of a kick from (QX, QY)/(1 + delta) held
+ * fixed (src/csbend.c:1627-1656, src/multipole.c:1359-1389): the momenta of
+ * the merged bodies.  So radiation leaves px and py alone and moves 1 + delta
+ * between the kicks, and its path factor sqrt(1 + x'^2 + y'^2) is the 1/pz of
+ * the drift that follows.  With ISR the deviates are most of a kick's work
+ * (10 integer rounds, a logarithm, a root and a cosine).  FODO ring with
+ * radiation and ISR in every magnet, RF and wake, 2e5 particles: 46 ms per
+ * turn through the general bodies, 18.6 through these. */
+
+/* trk_isr_gauss with cos(2 pi u) by cospi, exact in its reduction.  Out of line:
+ * inlined into the bodies to run beside the drifts' chain it was 10 % slower
+ * (spills, and three times the loop's code). */
+__device__ __noinline__ double isr_deviate(unsigned long long seed, unsigned id, unsigned pass, unsigned elem,
+                                           unsigned kick, double limit) {
+  for (unsigned attempt = 0; attempt < 64; attempt++) {
+    uint32_t c[4] = {id, pass, elem, (kick << 6) | attempt};
+    trk_philox4x32_10(c, (uint32_t)seed, (uint32_t)(seed >> 32));
+    const double u1 = trk_u53(c[0], c[1]), u2 = trk_u53(c[2], c[3]);
+    const double g = sqrt_fast(-2.0 * log(u1)) * cospi(2.0 * u2);
+    if (!(limit > 0) || fabs(g) <= limit)
+      return g;
+  }
+  return 0.0;
+}
+
+/* 1/opd after a relative change e of opd: 1 + e + e^2 + e^3 (the bodies accept
+ * changes of 1e-4 over the element) */
+__device__ __forceinline__ double rcp_update(double opd, double iopd) {
+  const double e = fma(-opd, iopd, 1.0);
+  return fma(iopd, fma(e, fma(e, e, e), e), iopd);
+}
+
+/* path length scaled to the new velocity: beta(P1) s / beta(P0) */
+__device__ __forceinline__ double beta_of(double p) { return p / sqrt(sqr(p) + 1); }
+
+template <int ORDER>
+__device__ __forceinline__ bool mult1_radiating(const trk_op *__restrict__ op, Part &p, double Po,
+                                                const trk_aperture *__restrict__ ap, const IsrKey &key) {
+  const double *d = op->d;
+  const int n_parts = __ldg(&op->i[0]), flags = __ldg(&op->i[6]);
+  const bool isr = (flags & MF_ISR) && !(key.single && (flags & MF_ISR1OFF));
+  const double len = __ldg(&d[MD_DRIFT]), rad = __ldg(&d[MD_RAD]) * len;
+  const double isr_c = isr ? __ldg(&d[MD_ISR]) * sqrt_fast(len * (1.0 / 3)) : 0;
+  /* the field the kicks stand for: K/(kick fraction len) |(fx, fy)|, the same for all */
+  const double field = __ldg(&d[MD_KQ]) / (__ldg(&d[MD_KFRAC]) * len), field2 = field * field;
+  double D = p.dp, opd = 1 + D, iopd = rcp_fast(opd);
+  if (!momentum_plain(opd))
+    return false;
+  const double ss = fma(p.yp, p.yp, fma(p.xp, p.xp, 1.0));
+  const double r0 = rsqrt_fast(ss);
+  double x = p.x, y = p.y, px = p.xp * r0, py = p.yp * r0;
+  const double l0 = __ldg(&d[MD_DSH]), l1 = __ldg(&d[MD_DSH + 1]);
+  unsigned zm = 0, xm = hi_abs(x), ym = hi_abs(y);
+  double s = l0 * (ss * r0), v = 0;
+  x = fma(p.xp, l0, x);
+  y = fma(p.yp, l0, y);
+#pragma unroll 1
+  for (int i = 0; i < n_parts; i++) {
+#pragma unroll 1
+    for (int j = 0; j < 3; j++) {
+      xm = max(xm, hi_abs(x));
+      ym = max(ym, hi_abs(y));
+      double fx, fy;
+      if (ORDER == 1) {
+        fy = x;
+        fx = y;
+      } else if (ORDER == 2) {
+        fy = 0.5 * fma(x, x, -y * y);
+        fx = x * y;
+      } else {
+        const double x2 = x * x, y2 = y * y;
+        fy = fma(-3.0, y2, x2) * x * (1.0 / 6);
+        fx = fma(3.0, x2, -y2) * y * (1.0 / 6);
+      }
+      const double K = __ldg(&d[MD_KQ + 3 * j]), k = K * iopd;
+      px = fma(-k, fy, px);
+      py = fma(k, fx, py);
+      const double z = fma(py, py, px * px);
+      zm = max(zm, (unsigned)__double2hiint(z));
+      v = sec_m1(z);
+      const double F2 = field2 * fma(fx, fx, fy * fy);
+      double loss = rad * __ldg(&d[MD_KFRAC + j]) * F2 * (1 + v);
+      if (isr) {
+        const double F = sqrt_fast(F2);
+        const double g = isr_deviate(key.seed, key.id, key.pass, key.elem, (unsigned)(i * 8 + j), key.limit);
+        loss = fma(isr_c * F * sqrt_fast(F * (1 + v)), g, loss);
+      }
+      D = fma(-(opd * opd), loss, D);
+      opd = 1 + D;
+      iopd = rcp_update(opd, iopd);
+      const double L = j < 2 ? l1 : i + 1 < n_parts ? 2 * l0 : l0, l = fma(L, v, L);
+      x = fma(px, l, x);
+      y = fma(py, l, y);
+      s += l;
+    }
+  }
+  xm = max(xm, hi_abs(x));
+  ym = max(ym, hi_abs(y));
+  if (!(zm < TRK_Z_HI && max(xm, ym) < TRK_COORD_HI && momentum_plain(opd) && fabs(D - p.dp) < 1e-4 * opd))
+    return false;
+  if (ap && !box_inside(above(xm), above(ym), ap))
+    return false;
+  p.x = x;
+  p.y = y;
+  p.xp = fma(px, v, px);
+  p.yp = fma(py, v, py);
+  if (__ldg(&d[MD_RAD]) != 0) {
+    const double b0 = beta_of(Po * (1 + p.dp)), b1 = beta_of(Po * opd);
+    p.s = b1 * (p.s / b0 + 2 * s / (b0 + b1));
+  } else
+    p.s += s;
+  p.dp = D;
+  return true;
+}
+
+__device__ __forceinline__ bool dipole_radiating(const trk_op *__restrict__ op, Part &p, double Po,
+                                                 const trk_aperture *__restrict__ ap, const IsrKey &key) {
+  const double *d = op->d;
+  const int nSlices = __ldg(&op->i[0]), flags = __ldg(&op->i[7]);
+  const bool isr = (flags & BF_ISR) && !(key.single && (flags & BF_ISR1OFF));
+  const double rho0 = __ldg(&d[BD_RHO0]), rhoinv = __ldg(&d[BD_RHOINV]), rad = __ldg(&d[BD_RAD]);
+  const double isr_c = isr ? __ldg(&d[BD_ISR]) * sqrt_fast(__ldg(&d[BD_SLICE]) * (1.0 / 3)) : 0;
+  double D = p.dp, opd = 1 + D, iopd = rcp_fast(opd);
+  if (!momentum_plain(opd))
+    return false;
+  const double r0 = rsqrt_fast(fma(p.yp, p.yp, fma(p.xp, p.xp, 1.0)));
+  const double py = p.yp * r0, py2 = py * py;
+  double px = p.xp * r0, X = p.x, F = 0, v = 0;
+  unsigned zm = 0, xm = hi_abs(X);
+  double R = rho0 + X;
+  /* 3 nSlices kicks, a drift before the first and after each */
+#pragma unroll 1
+  for (int k = -1, j = 2; k < 3 * nSlices; k++) {
+    if (k >= 0) {
+      j = j == 2 ? 0 : j + 1;
+      /* the second kick is what the first and third leave of the slice's
+       * whole (dipole_merged) */
+      const double ca = __ldg(&d[BD_C2]), c = j == 1 ? fma(-2.0, ca, __ldg(&d[BD_KT])) : ca;
+      px = fma(-(c * iopd), R, px);
+    }
+    const double z = fma(px, px, py2), h = cos_m1(z);
+    if (k >= 0) {
+      const double hs = (R * rhoinv) * (1 + sec_m1(z));
+      double loss = rad * __ldg(&d[BD_DS + j]) * hs;
+      if (isr) {
+        const double g =
+          isr_deviate(key.seed, key.id, key.pass, key.elem, (unsigned)(k / 3 * 8 + j), key.limit);
+        loss = fma(isr_c * sqrt_fast(hs), g, loss);
+      }
+      D = fma(-(opd * opd), loss, D);
+      opd = 1 + D;
+      iopd = rcp_update(opd, iopd);
+    }
+    const bool end = k < 0 || k == 3 * nSlices - 1;
+    const int S = end ? BD_SA : j == 2 ? BD_SA2 : BD_SA1, Cc = end ? BD_CA : j == 2 ? BD_CA2 : BD_CA + 1,
+              O = end ? BD_OMC : j == 2 ? BD_OMC2 : BD_OMC + 1;
+    const double sa = __ldg(&d[S]), ca = __ldg(&d[Cc]), omc = __ldg(&d[O]);
+    const double m = fma(-omc, h, fma(sa, px, omc));
+    px = fma(-sa, h, fma(ca, px, sa));
+    const double z1 = fma(px, px, py2);
+    v = sec_m1(z1);
+    zm = max(zm, max((unsigned)__double2hiint(z), (unsigned)__double2hiint(z1)));
+    const double u = fma(R, v, R);
+    X = fma(u, m, X);
+    F = fma(u, sa, F);
+    R = rho0 + X;
+    xm = max(xm, hi_abs(X));
+  }
+  const double Y = fma(py, F, p.y);
+  if (!(zm < TRK_Z_HI && max(xm, max(hi_abs(p.y), hi_abs(Y))) < TRK_COORD_HI && momentum_plain(opd) &&
+        fabs(D - p.dp) < 1e-4 * opd))
+    return false;
+  if (ap) {
+    const double xb = above(xm); /* as in dipole_merged */
+    if (!(xb < 0.125 * fabs(rho0)) || !box_inside(fma(2 * fabs(rho0), __ldg(&d[BD_OMC2]), xb),
+                                                  above(max(hi_abs(p.y), hi_abs(Y))), ap))
+      return false;
+  }
+  const double p0 = Po * (1 + p.dp), p1 = Po * opd;
+  p.s = p1 / sqrt(sqr(p1) + 1) * p.s / (p0 / sqrt(sqr(p0) + 1)) + F;
+  p.x = X;
+  p.y = Y;
+  p.xp = fma(px, v, px);
+  p.yp = fma(py, v, py);
+  p.dp = D;
+  return true;
+}
+
+/* The general kernel calls the special bodies out of line: inlined beside the
+ * general ones they took registers from both (radiating ring 5 % slower).
+ * lost < 0: not taken. */
+__device__ __noinline__ PartLoss radiating_call(const trk_op *__restrict__ op, Part p, double Po,
+                                                const trk_aperture *ap, IsrKey key) {
+  PartLoss r;
+  r.p = p;
+  bool done;
+  if (__ldg(&op->kind) == OPK_BEND)
+    done = dipole_radiating(op, r.p, Po, ap, key);
+  else {
+    const int order = __ldg(&op->i[4]) & 0xff;
+    done = order == 1   ? mult1_radiating<1>(op, r.p, Po, ap, key)
+           : order == 2 ? mult1_radiating<2>(op, r.p, Po, ap, key)
+                        : mult1_radiating<3>(op, r.p, Po, ap, key);
+  }
+  r.lost = done ? 0 : -1;
+  return r;
+}
+
+__device__ __noinline__ PartLoss merged_call(const trk_op *__restrict__ op, Part p, double Po, double z_start,
+                                             const trk_aperture *ap, const double *__restrict__ field) {
+  PartLoss r;
+  r.p = p;
+  const int kind = __ldg(&op->kind);
+  r.lost = !(kind == OPK_MULT1    ? op_mult1(op, r.p, Po, z_start, ap)
+             : kind == OPK_DIPOLE ? op_dipole(op, r.p, Po, z_start, ap)
+                                  : op_cfbend(op, r.p, Po, z_start, ap, field));
+  return r;
+}
 #endif
 
 /* ------------------------------------------------------ after-element */
@@ -3036,6 +3255,15 @@ __device__ __forceinline__ bool track_particle(const TrackArgs &a, const trk_op 
       const OpHead h = load_head(op, var);
       const trk_aperture *ap_in = h.ap_in >= 0 ? a.aps + h.ap_in : nullptr;
       bool ok = true;
+#if TRK_FAST
+      if (!LEAN && (h.kind == OPK_MULT1 || h.kind == OPK_DIPOLE || h.kind == OPK_CFBEND)) {
+        const PartLoss r = merged_call(op, p, a.Po, h.z_start, ap_in, a.field);
+        p = r.p;
+        if (!after_element(a, h, p, !r.lost, i, pass))
+          return false;
+        continue;
+      }
+#endif
       switch (h.kind) {
       case OPK_DRIFT:
         op_drift(op, p);
@@ -3046,21 +3274,23 @@ __device__ __forceinline__ bool track_particle(const TrackArgs &a, const trk_op 
         break;
       case OPK_MULT1:
 #if TRK_FAST
-        ok = op_mult1(op, p, a.Po, h.z_start, ap_in);
+        if (LEAN)
+          ok = op_mult1(op, p, a.Po, h.z_start, ap_in);
 #else
         ok = op_mult1_exact(op, p, a.Po, h.z_start, ap_in);
 #endif
         break;
       case OPK_DIPOLE:
 #if TRK_FAST
-        ok = op_dipole(op, p, a.Po, h.z_start, ap_in);
+        if (LEAN)
+          ok = op_dipole(op, p, a.Po, h.z_start, ap_in);
 #else
         ok = op_dipole_exact(op, p, a.Po, h.z_start, ap_in);
 #endif
         break;
       case OPK_CFBEND:
 #if TRK_FAST
-        if (LEAN != 1)
+        if (LEAN == 2)
           ok = op_cfbend(op, p, a.Po, h.z_start, ap_in, a.field);
 #else
         if (LEAN != 1) /* flavour 1 lattices hold no combined-function bend */
@@ -3080,6 +3310,15 @@ __device__ __forceinline__ bool track_particle(const TrackArgs &a, const trk_op 
           key.elem = (unsigned int)k;
           key.limit = a.isr_limit;
           key.single = a.n == 1;
+#if TRK_FAST
+          if (__ldg(&op->i[h.kind == OPK_MULT ? 6 : 7]) & (h.kind == OPK_MULT ? MF_MERGED : BF_MERGED)) {
+            const PartLoss r = radiating_call(op, p, a.Po, ap_in, key);
+            if (r.lost == 0) {
+              p = r.p;
+              break;
+            }
+          }
+#endif
           if (h.kind == OPK_MULT)
             ok = op_mult(op, p, a.Po, h.z_start, ap_in, &key);
           else

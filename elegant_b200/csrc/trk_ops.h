@@ -50,6 +50,7 @@ enum trk_op_kind {
 #define MF_ISR1OFF 2048 /* ISR1PART=0: no ISR when a single particle is tracked */
 #define MF_FRINGE1 4096 /* KQUAD entrance fringe (EDGE1_EFFECTS > 0) */
 #define MF_FRINGE2 8192 /* KQUAD exit fringe (EDGE2_EFFECTS > 0) */
+#define MF_MERGED 16384 /* OPK_MULT1 but for radiation: the fast build's radiating body */
 
 /* bend flags (i[7]) */
 #define BF_ISR_ROUNDTRIP 1 /* reference's (1+DPoP) divide/multiply round trip */
@@ -61,7 +62,8 @@ enum trk_op_kind {
 #define BF_EXPAND 64   /* EXPAND_HAMILTONIAN: leading-order drift, (1+delta) coordinate factors */
 #define BF_RADE1 128   /* SYNCH_RAD with an entrance edge angle: delta pre-adjusted at the entrance */
 #define BF_RADE2 256   /* ... and post-adjusted at the exit */
-#define BF_MERGED 512  /* substep angles small enough for the fast build's merged body */
+#define BF_MERGED 512  /* substep angles small enough for the fast build's merged body (OPK_DIPOLE, OPK_CFBEND,
+                          and OPK_BEND that would be OPK_DIPOLE but for radiation) */
 #define BF_LINEAR 1024 /* combined function: midplane field linear in x, its slope constant (K1 only) */
 
 /* RF flags (i[3]) */
