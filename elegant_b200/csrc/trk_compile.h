@@ -37,18 +37,25 @@ struct CompiledLattice {
   bool has_cfbend = false; /* some op is a combined-function CSBEND (OPK_CFBEND) */
 };
 
-/* Launch shape of the tracking kernel when the caller names none, measured on
- * B200: fast build (128 threads, 6 blocks/SM; 80 registers) for lean
- * lattices, (128, 5; 102 registers) for lean lattices with combined-function
- * bends, whose body spills at 80 registers; parity build (128, 6) for lean
- * lattices without combined-function bends (the FODO ring with RF and wake:
- * 94.6 ms per turn of 1e6 particles against 104.6 ms at (128, 4) and
- * 95.6 ms at (256, 3)); (128, 4) otherwise. */
 /* lean kernel flavour of a compiled lattice: 0 general, 1 lean, 2 lean with
  * combined-function bends */
 inline int trk_lean_flavor(const CompiledLattice &c) { return c.lean ? (c.has_cfbend ? 2 : 1) : 0; }
 
-inline int trk_default_variant(bool fast, const CompiledLattice &c) {
+/* Launch shape of the tracking kernel when the caller names none, for np
+ * particles on sms SMs (ms per turn on B200, this rule's choice first):
+ *  - up to 4 warps a scheduler, 512 particles an SM, (128 threads, 4 blocks/SM):
+ *    more blocks would not be resident anyway, and 128 registers spill nothing
+ *    (FODO ring, 1e4 particles: 0.39 against 0.43 at (128, 6); parity build,
+ *    30,011 particles with sextupoles: 3.2 against 3.8);
+ *  - lean lattices without combined-function bends, (128, 6): FODO ring with RF
+ *    and wake, 1e6 particles, parity 57.7 against 61.1 at (128, 4), fast 7.65
+ *    against 7.97;
+ *  - fast build with combined-function bends, (128, 5), which their body needs
+ *    not to spill: achromat ring, 1e6 particles, 79.6 against 81.3 at (128, 6);
+ *  - (128, 4) otherwise. */
+inline int trk_default_variant(bool fast, const CompiledLattice &c, long np, int sms) {
+  if (np <= 512L * sms)
+    return 1;
   if (c.lean && (fast || !c.has_cfbend))
     return fast && c.has_cfbend ? 4 : 7;
   return 1;

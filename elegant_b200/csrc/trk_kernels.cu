@@ -2294,149 +2294,6 @@ __device__ __forceinline__ bool op_cfbend_fast(const trk_op *__restrict__ op, Pa
   p.dp = D;
   return true;
 }
-
-/* Two particles through one pure dipole with their substep chains
- * interleaved: the body of each particle is a serial dependency chain
- * (sqrt -> reciprocal -> update), so a thread that carries two independent
- * chains keeps the FP64 pipe busier at the same occupancy.  Same arithmetic
- * per particle as op_dipole_fast; a slice that produced a non-finite value is
- * re-run for that particle with the reference's per-substep loss checks. */
-struct DipoleState {
-  double X, QX, F, QY, Y0, opd, f2;
-  int done;
-  bool ok;
-};
-
-__device__ __forceinline__ void dipole_begin(DipoleState &q, const Part &p) {
-  q.opd = 1 + p.dp;
-  const double r = q.opd * rsqrt_fast(fma(p.yp, p.yp, fma(p.xp, p.xp, 1.0)));
-  q.X = p.x;
-  q.Y0 = p.y;
-  q.QX = p.xp * r;
-  q.QY = p.yp * r;
-  q.F = 0;
-  q.f2 = q.opd * q.opd - q.QY * q.QY;
-  q.done = 0;
-}
-
-__device__ __forceinline__ void dipole_step(DipoleState &q, double rho0, double sa, double ca, double omc) {
-  const double fc = sqrt_nan(fma(-q.QX, q.QX, q.f2));
-  const double saq = sa * q.QX;
-  const double u = div_fast(rho0 + q.X, fma(ca, fc, -saq));
-  q.QX = fma(sa, fc, ca * q.QX);
-  q.F = fma(u, sa, q.F);
-  q.X = fma(u, fma(omc, fc, saq), q.X);
-}
-
-__device__ __forceinline__ bool dipole_finish(DipoleState &q, Part &p, const double *__restrict__ d, int nSlices,
-                                              double Po, double z_start, const trk_aperture *ap) {
-  double dz_lost = 0;
-  const double Y = q.Y0 + q.QY * q.F;
-  bool ok = q.ok;
-  if (ok) {
-    dz_lost = nSlices * __ldg(&d[BD_SLICE]);
-    if (ap && !check_aperture(q.X, Y, ap, false, 1.0, 0.0))
-      ok = false;
-  } else
-    for (int k = 0; k < q.done; k++)
-      dz_lost += __ldg(&d[BD_DSH + (k & 3)]);
-  const double f = rsqrt_fast(q.opd * q.opd - q.QX * q.QX - q.QY * q.QY);
-  p.x = q.X;
-  p.y = Y;
-  p.xp = q.QX * f;
-  p.yp = q.QY * f;
-  if (!ok) {
-    p.s = z_start + dz_lost;
-    p.dp = Po * q.opd; /* Po * (1 + delta) */
-    return false;
-  }
-  p.s += q.opd * q.F;
-  return true;
-}
-
-/* one slice for one particle with the reference's loss checks (rare path) */
-__device__ __forceinline__ void dipole_slice_checked(DipoleState &q, const double *__restrict__ d, double rho0) {
-  const SliceState r = dipole_slice_redo(d, 4, rho0, q.f2, q.X, q.QX, q.F, q.done);
-  q.ok = r.ok;
-  q.X = r.X;
-  q.QX = r.QX;
-  q.F = r.F;
-  q.done = r.done;
-}
-
-__device__ __forceinline__ void op_dipole_fast2(const trk_op *__restrict__ op, Part &p0, Part &p1, bool &ok0,
-                                                bool &ok1, double Po, double z_start, const trk_aperture *ap) {
-  const double *d = op->d;
-  const int nSlices = __ldg(&op->i[0]);
-  const double rho0 = __ldg(&d[BD_RHO0]);
-  DipoleState q0, q1;
-  dipole_begin(q0, p0);
-  dipole_begin(q1, p1);
-  q0.ok = ok0;
-  q1.ok = ok1;
-  for (int i = 0; i < nSlices; i++) {
-    if (ap) {
-      if (q0.ok && !check_aperture(q0.X, q0.Y0 + q0.QY * q0.F, ap, false, 1.0, 0.0))
-        q0.ok = false;
-      if (q1.ok && !check_aperture(q1.X, q1.Y0 + q1.QY * q1.F, ap, false, 1.0, 0.0))
-        q1.ok = false;
-    }
-    if (!(q0.f2 > 0))
-      q0.ok = false;
-    if (!(q1.f2 > 0))
-      q1.ok = false;
-    if (!q0.ok && !q1.ok)
-      break;
-    const double X0a = q0.X, QX0a = q0.QX, F0a = q0.F;
-    const double X0b = q1.X, QX0b = q1.QX, F0b = q1.F;
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-      const double sa = __ldg(&d[BD_SA + j]), ca = __ldg(&d[BD_CA + j]);
-      const double omc = __ldg(&d[BD_OMC + j]);
-      dipole_step(q0, rho0, sa, ca, omc);
-      dipole_step(q1, rho0, sa, ca, omc);
-      if (j == 3)
-        break;
-      const double c1 = __ldg(&d[BD_C1 + j]), c2 = __ldg(&d[BD_C2 + j]);
-      q0.QX = fma(-c2, q0.X, q0.QX - c1);
-      q1.QX = fma(-c2, q1.X, q1.QX - c1);
-    }
-    if (q0.ok) {
-      if (isfinite(q0.X + q0.QX + q0.F))
-        q0.done += 4;
-      else {
-        q0.X = X0a;
-        q0.QX = QX0a;
-        q0.F = F0a;
-        dipole_slice_checked(q0, d, rho0);
-      }
-    } else {
-      /* lost: keep the coordinates where the loss was found */
-      q0.X = X0a;
-      q0.QX = QX0a;
-      q0.F = F0a;
-    }
-    if (q1.ok) {
-      if (isfinite(q1.X + q1.QX + q1.F))
-        q1.done += 4;
-      else {
-        q1.X = X0b;
-        q1.QX = QX0b;
-        q1.F = F0b;
-        dipole_slice_checked(q1, d, rho0);
-      }
-    } else {
-      /* lost: keep the coordinates where the loss was found */
-      q1.X = X0b;
-      q1.QX = QX0b;
-      q1.F = F0b;
-    }
-  }
-  if (ok0)
-    ok0 = dipole_finish(q0, p0, d, nSlices, Po, z_start, ap);
-  if (ok1)
-    ok1 = dipole_finish(q1, p1, d, nSlices, Po, z_start, ap);
-}
 #endif
 
 #if TRK_FAST
@@ -3369,84 +3226,6 @@ __global__ void __launch_bounds__(BLOCK, MINB) track_kernel(TrackArgs a) {
   }
 }
 
-#if TRK_FAST
-__device__ __forceinline__ bool lean_op(const TrackArgs &a, const trk_op *__restrict__ op, const OpHead &h, Part &p,
-                                        const trk_aperture *ap_in) {
-  const double z_start = h.z_start;
-  switch (h.kind) {
-  case OPK_DRIFT:
-    op_drift(op, p);
-    return true;
-  case OPK_EDRIFT:
-  case OPK_RFDRIFT:
-    exact_drift(p, __ldg(&op->d[DD_L]));
-    return true;
-  case OPK_MULT1:
-    return op_mult1_fast(op, p, a.Po, z_start, ap_in);
-  case OPK_DIPOLE:
-    return op_dipole_fast(op, p, a.Po, z_start, ap_in);
-  case OPK_CFBEND:
-    return op_cfbend_fast(op, p, a.Po, z_start, ap_in, a.field);
-  case OPK_RF:
-    return op_rf(op, p, a.Po, h.z_end, a.rf_phase, a.rf_tave);
-  default:
-    return true;
-  }
-}
-
-/* Two particles per thread (lean lattices, fast build): particles i and
- * i + BLOCK of the block's tile. */
-template <int BLOCK, int MINB>
-__global__ void __launch_bounds__(BLOCK, MINB) track_kernel2(TrackArgs a) {
-  const long tile = 2L * BLOCK;
-  const long n = a.live ? __ldg(a.live_n) : a.n;
-  for (long base = (long)blockIdx.x * tile; base < n; base += (long)gridDim.x * tile) {
-    const long k0 = base + threadIdx.x, k1 = k0 + BLOCK;
-    const long i0 = k0 < n && a.live ? __ldg(&a.live[k0]) : k0;
-    const long i1 = k1 < n && a.live ? __ldg(&a.live[k1]) : k1;
-    bool al0 = k0 < n && a.lost_pass[i0] < 0;
-    bool al1 = k1 < n && a.lost_pass[i1] < 0;
-    if (!al0 && !al1)
-      continue;
-    Part p0, p1;
-    if (al0)
-      load_part(a, i0, p0);
-    else
-      p0 = Part{0, 0, 0, 0, 0, 0};
-    if (al1)
-      load_part(a, i1, p1);
-    else
-      p1 = Part{0, 0, 0, 0, 0, 0};
-    const bool was0 = al0, was1 = al1;
-    for (long pass = a.pass_begin; pass < a.pass_end && (al0 || al1); pass++) {
-      const int var = (pass == a.fresh_pass) ? 0 : 1;
-      for (int k = a.op_begin; k < a.op_end && (al0 || al1); k++) {
-        const trk_op *op = a.ops + k;
-        const OpHead h = load_head(op, var);
-        const trk_aperture *ap_in = h.ap_in >= 0 ? a.aps + h.ap_in : nullptr;
-        bool ok0 = al0, ok1 = al1;
-        if (h.kind == OPK_DIPOLE) {
-          op_dipole_fast2(op, p0, p1, ok0, ok1, a.Po, h.z_start, ap_in);
-        } else {
-          if (al0)
-            ok0 = lean_op(a, op, h, p0, ap_in);
-          if (al1)
-            ok1 = lean_op(a, op, h, p1, ap_in);
-        }
-        if (al0)
-          al0 = after_element(a, h, p0, ok0, i0, pass);
-        if (al1)
-          al1 = after_element(a, h, p1, ok1, i1, pass);
-      }
-    }
-    if (was0)
-      store_part(a, i0, p0);
-    if (was1)
-      store_part(a, i1, p1);
-  }
-}
-#endif
-
 /* computeTimeCoordinatesOnly (src/trwake.c:519-527), rounded step by step
  * in both builds so the statistics, binning and kick kernels agree. */
 __device__ __forceinline__ double wake_time(double Po, double dp, double s) {
@@ -4277,20 +4056,6 @@ static void launch_track_t(const TrackArgs &a, int variant, int grid, int block,
 }
 
 void launch_track(const TrackArgs &a, int variant, int lean, long n, int max_blocks, cudaStream_t st) {
-#if TRK_FAST
-  if (lean && (variant == 5 || variant == 6)) {
-    long g = (n + 2 * 128 - 1) / (2 * 128);
-    if (g < 1)
-      g = 1;
-    if (g > max_blocks)
-      g = max_blocks;
-    if (variant == 5)
-      track_kernel2<128, 3><<<(int)g, 128, 0, st>>>(a);
-    else
-      track_kernel2<128, 2><<<(int)g, 128, 0, st>>>(a);
-    return;
-  }
-#endif
   if (variant == 5 || variant == 6 || variant < 0 || variant >= TRK_N_VARIANTS)
     variant = 1;
   const int block = track_variant_block(variant);

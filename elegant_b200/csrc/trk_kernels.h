@@ -15,7 +15,7 @@
 
 /* launch shapes of the tracking kernel (trk_run.variant):
  * 0 (128 threads, 1 block/SM min), 1 (128, 4), 2 (256, 2), 3 (64, 8), 4 (128, 5),
- * 5 and 6: two particles per thread (128, 3) / (128, 2), lean lattices in the fast build,
+ * 5 and 6: run as 1 (they were two particles per thread, which the merged bodies overtook),
  * 7 (128, 6), 8 (256, 3) */
 #define TRK_N_VARIANTS 9
 
