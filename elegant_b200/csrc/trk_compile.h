@@ -49,7 +49,7 @@ inline int trk_lean_flavor(const CompiledLattice &c) { return c.lean ? (c.has_cf
  *    30,011 particles with sextupoles: 3.2 against 3.8);
  *  - lean lattices without combined-function bends, (128, 6): FODO ring with RF
  *    and wake, 1e6 particles, parity 57.7 against 61.1 at (128, 4), fast 7.65
- *    against 7.97;
+ *    against 7.97 (before the merged bodies left the aperture to the checked ones);
  *  - fast build with combined-function bends, (128, 5), which their body needs
  *    not to spill: achromat ring, 1e6 particles, 79.6 against 81.3 at (128, 6);
  *  - (128, 4) otherwise. */

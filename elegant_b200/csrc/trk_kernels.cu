@@ -76,6 +76,12 @@ struct PartLoss {
 __device__ __forceinline__ unsigned hi_abs(double v) { return (unsigned)__double2hiint(v) & 0x7fffffffu; }
 __device__ __forceinline__ bool finite2(double u, double v) { return max(hi_abs(u), hi_abs(v)) < 0x7ff00000u; }
 
+/* the high words of the largest |x| and |y| seen */
+__device__ __forceinline__ void box_add(unsigned *box, double x, double y) {
+  box[0] = max(box[0], hi_abs(x));
+  box[1] = max(box[1], hi_abs(y));
+}
+
 #if TRK_FAST
 /* Reciprocal and square root for the fast build: the hardware approximation
  * y0 (about 20 correct bits) and one third-order correction from the series
@@ -273,7 +279,7 @@ template <int ORDER>
 __device__ __forceinline__ int mult_body_fast(const double *__restrict__ d, int n_parts, const trk_aperture *ap,
                                               bool aptilt, double apc, double aps, double mdx, double mdy, double &x,
                                               double &xp, double &y, double &yp, double &s, double &qx, double &qy,
-                                              const double dp, int &done) {
+                                              const double dp, int &done, unsigned *box = nullptr) {
   const double opd2 = (1 + dp) * (1 + dp);
   /* path-length factor sqrt(1 + xp^2 + yp^2): once from the entry slopes,
    * then (1+delta) / sqrt((1+delta)^2 - qx^2 - qy^2) from each slope update,
@@ -283,6 +289,8 @@ __device__ __forceinline__ int mult_body_fast(const double *__restrict__ d, int 
   for (int i_kick = 0; i_kick < n_parts; i_kick++) {
     if (ap && !check_aperture(x + mdx, y + mdy, ap, aptilt, apc, aps))
       return 1;
+    if (box)
+      box_add(box, x, y);
 #pragma unroll
     for (int step = 0; step < 4; step++) {
       const double dsh = __ldg(&d[MD_DSH + step]);
@@ -315,6 +323,8 @@ __device__ __forceinline__ int mult_body_fast(const double *__restrict__ d, int 
   }
   if (ap && !check_aperture(x + mdx, y + mdy, ap, aptilt, apc, aps))
     return 1;
+  if (box)
+    box_add(box, x, y);
   return 0;
 }
 #endif
@@ -973,7 +983,7 @@ template <int NSUB>
 __device__ __forceinline__ bool bend_dipole_fast(const double *__restrict__ d, int nSlices, int nSub_rt, double rho0,
                                                  const trk_aperture *ap, bool aptilt, double apc, double aps,
                                                  double &X, double &QX, double &Y, const double QY, const double D,
-                                                 double &dist, int &done) {
+                                                 double &dist, int &done, unsigned *box = nullptr) {
   const int nSub = NSUB > 0 ? NSUB : nSub_rt;
   const double opd = 1 + D;
   const double f2 = opd * opd - QY * QY;
@@ -986,6 +996,8 @@ __device__ __forceinline__ bool bend_dipole_fast(const double *__restrict__ d, i
       ok = false;
       break;
     }
+    if (box)
+      box_add(box, X, Y0 + QY * F);
     if (!(f2 > 0)) {
       ok = false;
       break;
@@ -1101,7 +1113,8 @@ __device__ __noinline__ CfState cf_slice_redo(const double *__restrict__ d, cons
 
 __device__ __forceinline__ bool bend_cf_fast(const double *__restrict__ d, const double *__restrict__ fxy,
                                              int nSlices, double rho0, const trk_aperture *ap, double &X, double &QX,
-                                             double &Y, double &QY, const double D, double &dist, int &done) {
+                                             double &Y, double &QY, const double D, double &dist, int &done,
+                                             unsigned *box = nullptr) {
   const double opd = 1 + D;
   bool ok = true;
   dist = 0;
@@ -1111,6 +1124,8 @@ __device__ __forceinline__ bool bend_cf_fast(const double *__restrict__ d, const
       ok = false;
       break;
     }
+    if (box)
+      box_add(box, X, Y);
     const double *dd = d;
     asm volatile("" : "+l"(dd));
     const double X0 = X, QX0 = QX, Y0 = Y, QY0 = QY, S0 = dist;
@@ -2155,7 +2170,7 @@ __device__ __forceinline__ bool op_rf(const trk_op *__restrict__ op, Part &p, do
  * the reference before the body (src/multipole.c:1190-1228) is an identity
  * in exact arithmetic and is skipped. */
 __device__ __forceinline__ bool op_mult1_fast(const trk_op *__restrict__ op, Part &p, double Po, double z_start,
-                                              const trk_aperture *ap) {
+                                              const trk_aperture *ap, unsigned *box = nullptr) {
   const int n_parts = __ldg(&op->i[0]);
   const int order = __ldg(&op->i[4]) & 0xff;
   const int flags = __ldg(&op->i[6]);
@@ -2174,11 +2189,11 @@ __device__ __forceinline__ bool op_mult1_fast(const trk_op *__restrict__ op, Par
     double qx = xp * r, qy = yp * r;
     int done = 0, rc;
     if (order == 1)
-      rc = mult_body_fast<1>(d, n_parts, ap, aptilt, apc, aps, 0.0, 0.0, x, xp, y, yp, s, qx, qy, dp, done);
+      rc = mult_body_fast<1>(d, n_parts, ap, aptilt, apc, aps, 0.0, 0.0, x, xp, y, yp, s, qx, qy, dp, done, box);
     else if (order == 2)
-      rc = mult_body_fast<2>(d, n_parts, ap, aptilt, apc, aps, 0.0, 0.0, x, xp, y, yp, s, qx, qy, dp, done);
+      rc = mult_body_fast<2>(d, n_parts, ap, aptilt, apc, aps, 0.0, 0.0, x, xp, y, yp, s, qx, qy, dp, done, box);
     else
-      rc = mult_body_fast<3>(d, n_parts, ap, aptilt, apc, aps, 0.0, 0.0, x, xp, y, yp, s, qx, qy, dp, done);
+      rc = mult_body_fast<3>(d, n_parts, ap, aptilt, apc, aps, 0.0, 0.0, x, xp, y, yp, s, qx, qy, dp, done, box);
     if (rc) {
       for (int k = 0; k < done; k++)
         dzLoss += __ldg(&d[MD_DSH + (k & 3)]);
@@ -2223,7 +2238,7 @@ __device__ __forceinline__ bool op_mult1_fast(const trk_op *__restrict__ op, Par
  * no misalignment and no edge kick (src/csbend.c:654-1434), body by
  * bend_dipole_fast. */
 __device__ __forceinline__ bool op_dipole_fast(const trk_op *__restrict__ op, Part &p, double Po, double z_start,
-                                               const trk_aperture *ap) {
+                                               const trk_aperture *ap, unsigned *box = nullptr) {
   const double *d = op->d;
   const int nSlices = __ldg(&op->i[0]);
   const double rho0 = __ldg(&d[BD_RHO0]);
@@ -2233,7 +2248,9 @@ __device__ __forceinline__ bool op_dipole_fast(const trk_op *__restrict__ op, Pa
   const double QY = p.yp * r;
   double dist = 0;
   int done = 0;
-  bool ok = bend_dipole_fast<4>(d, nSlices, 4, rho0, ap, false, 1.0, 0.0, X, QX, Y, QY, D, dist, done);
+  bool ok = bend_dipole_fast<4>(d, nSlices, 4, rho0, ap, false, 1.0, 0.0, X, QX, Y, QY, D, dist, done, box);
+  if (box)
+    box_add(box, X, Y);
   double dz_lost = 0;
   if (ok) {
     dz_lost = nSlices * __ldg(&d[BD_SLICE]);
@@ -2261,7 +2278,8 @@ __device__ __forceinline__ bool op_dipole_fast(const trk_op *__restrict__ op, Pa
  * dipole (normal field expansion of order 4) with no misalignment and no edge
  * kick (src/csbend.c:654-1434), body by bend_cf_fast. */
 __device__ __forceinline__ bool op_cfbend_fast(const trk_op *__restrict__ op, Part &p, double Po, double z_start,
-                                               const trk_aperture *ap, const double *__restrict__ field) {
+                                               const trk_aperture *ap, const double *__restrict__ field,
+                                               unsigned *box = nullptr) {
   const double *d = op->d;
   const int nSlices = __ldg(&op->i[0]);
   const double *fxy = field + __ldg(&op->i[4]);
@@ -2271,7 +2289,9 @@ __device__ __forceinline__ bool op_cfbend_fast(const trk_op *__restrict__ op, Pa
   double X = p.x, Y = p.y, QX = p.xp * r, QY = p.yp * r;
   double dist = 0;
   int done = 0;
-  bool ok = bend_cf_fast(d, fxy, nSlices, rho0, ap, X, QX, Y, QY, D, dist, done);
+  bool ok = bend_cf_fast(d, fxy, nSlices, rho0, ap, X, QX, Y, QY, D, dist, done, box);
+  if (box)
+    box_add(box, X, Y);
   double dz_lost = 0;
   if (ok) {
     dz_lost = nSlices * __ldg(&d[BD_SLICE]);
@@ -2312,16 +2332,14 @@ __device__ __forceinline__ bool op_cfbend_fast(const trk_op *__restrict__ op, Pa
  *    root per substep, and a chain of multiply-adds instead of two dependent
  *    hardware approximations.
  * The loss conditions of the element (undefined slopes, |QX| > f, limits on
- * coordinates and slopes, the per-slice aperture) are excluded by bounds kept
- * on the way as integer maxima of high words (ALU pipe): a particle that
- * comes near any of them leaves the body unchanged and takes the checked one
+ * coordinates and slopes) are excluded by a bound on z kept on the way as an
+ * integer maximum of high words (ALU pipe) and by the ends' positions: a
+ * particle near any of them leaves the body unchanged and takes the checked one
  * (op_mult1_fast and so on), which locates the loss as the reference does.
  * Bound by FP64 issue and by the length of the substep's chain (13 of its 17
  * operations).  Measured against the checked bodies alone, ms per turn: FODO
- * ring with RF and wake, 1e6 particles, 11.4 -> 7.6; achromat ring, 2e6, 250
- * -> 158; FODO ring, 1e4 particles, 0.67 -> 0.41; dynamic-aperture grids over
- * 24 seeds, where the checked bodies divide for the aperture in every slice,
- * 101 -> 46 for 32 turns. */
+ * ring with RF and wake, 1e6 particles, 11.4 -> 7.5; achromat ring, 2e6, 250
+ * -> 149; FODO ring, 1e4 particles, 0.67 -> 0.36. */
 
 /* Coefficients: the power series, its first omitted term economized over
  * [0, b], b = 2^-12 (z^4 replaced by z^4 - b^4 T4*(z/b)/128 without the
@@ -2377,22 +2395,19 @@ __device__ __forceinline__ double kick_over(double k, double opd, double iopd) {
  * the kick, 9 of the drift (13 and 15 in the unmerged body, with a reciprocal
  * square root). */
 template <int ORDER>
-__device__ __forceinline__ bool mult1_merged(const double *__restrict__ d, int n_parts, Part &p,
-                                             const trk_aperture *__restrict__ ap) {
+__device__ __forceinline__ bool mult1_merged(const double *__restrict__ d, int n_parts, Part &p) {
   const double opd = 1 + p.dp, iopd = rcp_fast(opd);
   const double ss = fma(p.yp, p.yp, fma(p.xp, p.xp, 1.0));
   const double r0 = rsqrt_fast(ss);
   double x = p.x, y = p.y, px = p.xp * r0, py = p.yp * r0;
   const double l0 = __ldg(&d[MD_DSH]), l1 = __ldg(&d[MD_DSH + 1]);
   const double ka = kick_over(__ldg(&d[MD_KQ]), opd, iopd), kb = kick_over(__ldg(&d[MD_KQ + 3]), opd, iopd);
-  unsigned zm = 0, xm = hi_abs(x), ym = hi_abs(y);
+  unsigned zm = 0;
   double s = l0 * (ss * r0), v = 0; /* first drift: slopes xp, sqrt(1 + xp^2 + yp^2) */
   x = fma(p.xp, l0, x);
   y = fma(p.yp, l0, y);
 #define TRK_KICK(K)                                                                                          \
   {                                                                                                          \
-    xm = max(xm, hi_abs(x));                                                                                 \
-    ym = max(ym, hi_abs(y));                                                                                 \
     if (ORDER == 1) {                                                                                        \
       px = fma(-(K), x, px);                                                                                 \
       py = fma((K), y, py);                                                                                  \
@@ -2426,12 +2441,8 @@ __device__ __forceinline__ bool mult1_merged(const double *__restrict__ d, int n
   }
 #undef TRK_KICK
 #undef TRK_DRIFT
-  xm = max(xm, hi_abs(x));
-  ym = max(ym, hi_abs(y));
-  if (!(zm < TRK_Z_HI && max(xm, ym) < TRK_COORD_HI && momentum_plain(opd)))
-    return false;
-  /* every slice boundary lies on a straight segment between these points */
-  if (ap && !box_inside(above(xm), above(ym), ap))
+  if (!(zm < TRK_Z_HI && max(max(hi_abs(x), hi_abs(y)), max(hi_abs(p.x), hi_abs(p.y))) < TRK_COORD_HI &&
+        momentum_plain(opd)))
     return false;
   p.x = x;
   p.y = y;
@@ -2448,8 +2459,7 @@ __device__ __forceinline__ bool mult1_merged(const double *__restrict__ d, int n
  * is px -= k R with R = rho0 + X, k = ds/(rho_actual rho0 (1 + delta)).  17
  * operations per kick and drift (20 with a root and a reciprocal in the
  * unmerged body). */
-__device__ __forceinline__ bool dipole_merged(const double *__restrict__ d, int nSlices, Part &p,
-                                              const trk_aperture *__restrict__ ap) {
+__device__ __forceinline__ bool dipole_merged(const double *__restrict__ d, int nSlices, Part &p) {
   const double rho0 = __ldg(&d[BD_RHO0]);
   const double opd = 1 + p.dp, iopd = rcp_fast(opd);
   const double r0 = rsqrt_fast(fma(p.yp, p.yp, fma(p.xp, p.xp, 1.0)));
@@ -2459,7 +2469,7 @@ __device__ __forceinline__ bool dipole_merged(const double *__restrict__ d, int 
   const double kb = fma(-2.0, ka, kick_over(__ldg(&d[BD_KT]), opd, iopd));
   const double s1 = __ldg(&d[BD_SA1]), c1 = __ldg(&d[BD_CA + 1]), m1 = __ldg(&d[BD_OMC + 1]);
   const double s2 = __ldg(&d[BD_SA2]), c2 = __ldg(&d[BD_CA2]), m2 = __ldg(&d[BD_OMC2]);
-  unsigned zm = 0, xm = hi_abs(X);
+  unsigned zm = 0;
   double R = rho0 + X;
 #define TRK_DRIFT(SA, CA, OMC)                                                                               \
   {                                                                                                          \
@@ -2473,7 +2483,6 @@ __device__ __forceinline__ bool dipole_merged(const double *__restrict__ d, int 
     X = fma(u, m, X);                                                                                        \
     F = fma(u, (SA), F);                                                                                     \
     R = rho0 + X;                                                                                            \
-    xm = max(xm, hi_abs(X));                                                                                 \
   }
   {
     const double s0 = __ldg(&d[BD_SA]), c0 = __ldg(&d[BD_CA]), m0 = __ldg(&d[BD_OMC]);
@@ -2494,17 +2503,8 @@ __device__ __forceinline__ bool dipole_merged(const double *__restrict__ d, int 
   }
 #undef TRK_DRIFT
   const double Y = fma(py, F, p.y);
-  if (!(zm < TRK_Z_HI && max(xm, max(hi_abs(p.y), hi_abs(Y))) < TRK_COORD_HI && momentum_plain(opd)))
+  if (!(zm < TRK_Z_HI && max(max(hi_abs(X), hi_abs(Y)), max(hi_abs(p.x), hi_abs(p.y))) < TRK_COORD_HI && momentum_plain(opd)))
     return false;
-  if (ap) {
-    /* a slice boundary lies on a chord between two of these points, at most
-     * R (1 - cos a) nearer the centre; with |X| below rho0/8 the path grows
-     * from slice to slice, so Y stays between its ends */
-    const double xb = above(xm);
-    if (!(xb < 0.125 * fabs(rho0)) ||
-        !box_inside(fma(2 * fabs(rho0), m2, xb), above(max(hi_abs(p.y), hi_abs(Y))), ap))
-      return false;
-  }
   p.x = X;
   p.y = Y;
   p.xp = fma(px, v, px);
@@ -2517,14 +2517,14 @@ __device__ __forceinline__ bool dipole_merged(const double *__restrict__ d, int 
  * LIN: K1 only, the midplane field linear in x and its slope constant. */
 template <bool LIN>
 __device__ __forceinline__ bool cfbend_merged(const double *__restrict__ d, const double *__restrict__ fxy, int nSlices,
-                                              Part &p, const trk_aperture *__restrict__ ap) {
+                                              Part &p) {
   const double rho0 = __ldg(&d[BD_RHO0]);
   const double opd = 1 + p.dp, iopd = rcp_fast(opd);
   const double r0 = rsqrt_fast(fma(p.yp, p.yp, fma(p.xp, p.xp, 1.0)));
   double px = p.xp * r0, py = p.yp * r0, X = p.x, Y = p.y, dist = 0, v = 0;
   const double ca = kick_over(__ldg(&d[BD_C2]), opd, iopd);
   const double cb = fma(-2.0, ca, kick_over(__ldg(&d[BD_KT]), opd, iopd));
-  unsigned zm = 0, xm = hi_abs(X), ym = hi_abs(Y);
+  unsigned zm = 0;
   double R = rho0 + X, py2 = py * py;
 #define CF_T(T, i, j) __ldg(&(T)[(i) * 11 + (j)])
 #define TRK_DRIFT(S, C, O)                                                                                   \
@@ -2541,8 +2541,6 @@ __device__ __forceinline__ bool cfbend_merged(const double *__restrict__ d, cons
     Y = fma(py, us, Y);                                                                                      \
     dist += us;                                                                                              \
     R = rho0 + X;                                                                                            \
-    xm = max(xm, hi_abs(X));                                                                                 \
-    ym = max(ym, hi_abs(Y));                                                                                 \
   }
 #define TRK_KICK(K)                                                                                          \
   {                                                                                                          \
@@ -2586,15 +2584,9 @@ __device__ __forceinline__ bool cfbend_merged(const double *__restrict__ d, cons
 #undef TRK_KICK
 #undef TRK_DRIFT
 #undef CF_T
-  if (!(zm < TRK_Z_HI && max(xm, ym) < TRK_COORD_HI && momentum_plain(opd)))
+  if (!(zm < TRK_Z_HI && max(max(hi_abs(X), hi_abs(Y)), max(hi_abs(p.x), hi_abs(p.y))) < TRK_COORD_HI &&
+        momentum_plain(opd)))
     return false;
-  if (ap) {
-    /* as in dipole_merged; Y runs along the same chords */
-    const double xb = above(xm);
-    if (!(xb < 0.125 * fabs(rho0)) ||
-        !box_inside(fma(2 * fabs(rho0), __ldg(&d[BD_OMC2]), xb), above(ym), ap))
-      return false;
-  }
   p.x = X;
   p.y = Y;
   p.xp = fma(px, v, px);
@@ -2605,10 +2597,23 @@ __device__ __forceinline__ bool cfbend_merged(const double *__restrict__ d, cons
 
 /* The checked bodies out of line for the particles the merged ones leave,
  * passed and returned by value (a reference would pin the caller's
- * coordinates in local memory). */
+ * coordinates in local memory).  All elements inside an aperture come here:
+ * particles near the dynamic aperture move chaotically, and any other order
+ * of rounding changes their tracks by up to 1e-4 of the beam after 32 turns,
+ * so aperture studies keep the unmerged arithmetic.  What they do not need is
+ * the test in every slice, with its divisions: the body runs without it and
+ * the box around the slice boundaries is tested in products; only a particle
+ * whose box is not clear of the aperture is taken through the tests. */
 __device__ __noinline__ PartLoss mult1_checked(const trk_op *__restrict__ op, Part p, double Po, double z_start,
                                                const trk_aperture *ap) {
   PartLoss r;
+  if (ap) {
+    unsigned box[2] = {0, 0};
+    r.p = p;
+    r.lost = !op_mult1_fast(op, r.p, Po, z_start, nullptr, box);
+    if (!r.lost && box_inside(above(box[0]), above(box[1]), ap))
+      return r;
+  }
   r.lost = !op_mult1_fast(op, p, Po, z_start, ap);
   r.p = p;
   return r;
@@ -2617,6 +2622,13 @@ __device__ __noinline__ PartLoss mult1_checked(const trk_op *__restrict__ op, Pa
 __device__ __noinline__ PartLoss dipole_checked(const trk_op *__restrict__ op, Part p, double Po, double z_start,
                                                 const trk_aperture *ap) {
   PartLoss r;
+  if (ap) {
+    unsigned box[2] = {0, 0};
+    r.p = p;
+    r.lost = !op_dipole_fast(op, r.p, Po, z_start, nullptr, box);
+    if (!r.lost && box_inside(above(box[0]), above(box[1]), ap))
+      return r;
+  }
   r.lost = !op_dipole_fast(op, p, Po, z_start, ap);
   r.p = p;
   return r;
@@ -2625,6 +2637,13 @@ __device__ __noinline__ PartLoss dipole_checked(const trk_op *__restrict__ op, P
 __device__ __noinline__ PartLoss cfbend_checked(const trk_op *__restrict__ op, Part p, double Po, double z_start,
                                                 const trk_aperture *ap, const double *__restrict__ field) {
   PartLoss r;
+  if (ap) {
+    unsigned box[2] = {0, 0};
+    r.p = p;
+    r.lost = !op_cfbend_fast(op, r.p, Po, z_start, nullptr, field, box);
+    if (!r.lost && box_inside(above(box[0]), above(box[1]), ap))
+      return r;
+  }
   r.lost = !op_cfbend_fast(op, p, Po, z_start, ap, field);
   r.p = p;
   return r;
@@ -2633,13 +2652,15 @@ __device__ __noinline__ PartLoss cfbend_checked(const trk_op *__restrict__ op, P
 __device__ __forceinline__ bool op_mult1(const trk_op *__restrict__ op, Part &p, double Po, double z_start,
                                          const trk_aperture *ap) {
   const int n_parts = __ldg(&op->i[0]), order = __ldg(&op->i[4]) & 0xff;
-  bool done;
-  if (order == 1)
-    done = mult1_merged<1>(op->d, n_parts, p, ap);
+  bool done = false;
+  if (ap)
+    ;
+  else if (order == 1)
+    done = mult1_merged<1>(op->d, n_parts, p);
   else if (order == 2)
-    done = mult1_merged<2>(op->d, n_parts, p, ap);
+    done = mult1_merged<2>(op->d, n_parts, p);
   else
-    done = mult1_merged<3>(op->d, n_parts, p, ap);
+    done = mult1_merged<3>(op->d, n_parts, p);
   if (done)
     return true;
   const PartLoss r = mult1_checked(op, p, Po, z_start, ap);
@@ -2649,7 +2670,7 @@ __device__ __forceinline__ bool op_mult1(const trk_op *__restrict__ op, Part &p,
 
 __device__ __forceinline__ bool op_dipole(const trk_op *__restrict__ op, Part &p, double Po, double z_start,
                                           const trk_aperture *ap) {
-  if ((__ldg(&op->i[7]) & BF_MERGED) && dipole_merged(op->d, __ldg(&op->i[0]), p, ap))
+  if (!ap && (__ldg(&op->i[7]) & BF_MERGED) && dipole_merged(op->d, __ldg(&op->i[0]), p))
     return true;
   const PartLoss r = dipole_checked(op, p, Po, z_start, ap);
   p = r.p;
@@ -2659,10 +2680,10 @@ __device__ __forceinline__ bool op_dipole(const trk_op *__restrict__ op, Part &p
 __device__ __forceinline__ bool op_cfbend(const trk_op *__restrict__ op, Part &p, double Po, double z_start,
                                           const trk_aperture *ap, const double *__restrict__ field) {
   const int flags = __ldg(&op->i[7]);
-  if (flags & BF_MERGED) {
+  if (!ap && (flags & BF_MERGED)) {
     const double *fxy = field + __ldg(&op->i[4]);
-    if ((flags & BF_LINEAR) ? cfbend_merged<true>(op->d, fxy, __ldg(&op->i[0]), p, ap)
-                            : cfbend_merged<false>(op->d, fxy, __ldg(&op->i[0]), p, ap))
+    if ((flags & BF_LINEAR) ? cfbend_merged<true>(op->d, fxy, __ldg(&op->i[0]), p)
+                            : cfbend_merged<false>(op->d, fxy, __ldg(&op->i[0]), p))
       return true;
   }
   const PartLoss r = cfbend_checked(op, p, Po, z_start, ap, field);
@@ -2843,7 +2864,10 @@ __device__ __forceinline__ bool dipole_radiating(const trk_op *__restrict__ op, 
         fabs(D - p.dp) < 1e-4 * opd))
     return false;
   if (ap) {
-    const double xb = above(xm); /* as in dipole_merged */
+    const double xb = above(xm);
+    /* a slice boundary lies on a chord between two of these points, at most
+     * R (1 - cos a) nearer the centre; with |X| below rho0/8 the path grows
+     * from slice to slice, so Y stays between its ends */
     if (!(xb < 0.125 * fabs(rho0)) || !box_inside(fma(2 * fabs(rho0), __ldg(&d[BD_OMC2]), xb),
                                                   above(max(hi_abs(p.y), hi_abs(Y))), ap))
       return false;
