@@ -1976,7 +1976,8 @@ static int adjoint_run(trk_context *ctx, const trk_lattice *const *lattices, int
   std::vector<int> op_dfield(std::max(nops, 1), -1);
   std::vector<double> dfield;
   std::vector<const trk_elem *> dfield_elem; /* the bend each table was formed for */
-  for (int k = 0; k < nops; k++) {
+  /* the kinds depend on parameter values, so every variant's records are looked at */
+  for (int k = 0; k < nops * nv; k++) {
     const trk_op &op = c.ops[k];
     switch (op.kind) {
     case OPK_NOP:
@@ -1994,26 +1995,33 @@ static int adjoint_run(trk_context *ctx, const trk_lattice *const *lattices, int
         return trk_set_error(TRK_ERR_UNSUPPORTED, "CSBEND with more than 32 slices in a gradient run");
       break;
     default:
-      return trk_set_error(TRK_ERR_UNSUPPORTED, "element %d: gradients cover DRIF, EDRIFT, KQUAD/KSEXT/KOCT "
-                           "(single order, no tilt or misalignment) and CSBEND (pure dipole or K1/K2 "
-                           "expansion, no misalignment or edge kick)", op.elem);
+      return trk_set_error(TRK_ERR_UNSUPPORTED, "variant %d, element %d: gradients cover DRIF, EDRIFT, KQUAD/KSEXT/"
+                           "KOCT (single order, no tilt or misalignment) and CSBEND (pure dipole or K1/K2 "
+                           "expansion, no misalignment or edge kick)", k / nops, op.elem);
     }
+  }
+  for (int k = 0; k < nops; k++) {
+    const trk_op &op = c.ops[k];
     const int pe = (op.elem >= 0 && op.elem < lattice->n) ? param_of_elem[op.elem] : -1;
     if (pe >= 0 && lattice->e[op.elem].type == TRK_CSBEND) {
       /* K1 and K2 of a bend: the kicks' field derivatives (a zero-angle
        * CSBEND is a drift, and USE_BN ignores K: zero gradient) */
-      if (op.kind != OPK_DIPOLE && op.kind != OPK_CFBEND)
+      bool any = false;
+      for (int v = 0; v < nv; v++) {
+        const int kind = c.ops[(size_t)v * nops + k].kind;
+        any = any || ((kind == OPK_DIPOLE || kind == OPK_CFBEND) && !TRK_P(&lattices[v]->e[op.elem], CSBEND_USE_BN));
+      }
+      if (!any)
         continue;
       const trk_elem *e0 = &lattices[0]->e[op.elem];
-      if (TRK_P(e0, CSBEND_USE_BN))
-        continue;
       static const int same[] = {P_CSBEND_L, P_CSBEND_ANGLE, P_CSBEND_FSE, P_CSBEND_FSE_DIPOLE,
-                                 P_CSBEND_FSE_QUADRUPOLE, P_CSBEND_NONLINEAR, P_CSBEND_EXPANSION_ORDER};
+                                 P_CSBEND_FSE_QUADRUPOLE, P_CSBEND_NONLINEAR, P_CSBEND_EXPANSION_ORDER,
+                                 P_CSBEND_USE_BN};
       for (int v = 1; v < nv; v++)
         for (int q : same)
           if (lattices[v]->e[op.elem].p[q] != e0->p[q])
             return trk_set_error(TRK_ERR_UNSUPPORTED, "element %d: CSBEND gradients need the variants to share "
-                                 "L, ANGLE, FSE* and the expansion settings", op.elem);
+                                 "L, ANGLE, FSE*, USE_BN and the expansion settings", op.elem);
       op_param[k] = pe;
       /* one table for bends that share everything it depends on */
       for (size_t m = 0; m < dfield_elem.size() && op_dfield[k] < 0; m++) {

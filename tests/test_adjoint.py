@@ -205,3 +205,20 @@ def test_adjoint_rejects_misaligned_bend():
         trk.load(configs.c5_beam(100, seed=98))
         with pytest.raises(RuntimeError):
             trk.adjoint(lat, 2, PC, W)
+
+
+@pytest.mark.parametrize("element, change", [("CSBEND", dict(DX=1e-4)), ("CSBEND", dict(TILT=0.01)),
+                                             ("CSBEND", dict(E1=0.01)), ("CSBEND", dict(SYNCH_RAD=1.0)),
+                                             ("CSBEND", dict(USE_BN=1.0)), ("KOCT", dict(DY=1e-4)),
+                                             ("KOCT", dict(SYNCH_RAD=1.0)), ("KQUAD", dict(TILT=0.01))])
+@pytest.mark.parametrize("first", [False, True])
+def test_adjoint_ensemble_rejects_elements_of_any_variant(element, change, first):
+    """One of two error seeds holds an element that gradients do not cover:
+    the batch is refused wherever that seed stands."""
+    lats = [_mba(), _mba()]
+    e = next(e for e in lats[0 if first else 1].elements if e[0] == element)
+    e[2].update(change)
+    with Tracker(0) as trk:
+        trk.load(configs.c5_beam(100, seed=98))
+        with pytest.raises(RuntimeError):
+            trk.adjoint_ensemble(lats, [50, 50], 2, PC, W)
