@@ -2049,13 +2049,33 @@ static int adjoint_run(trk_context *ctx, const trk_lattice *const *lattices, int
   }
   const long np = ctx->np, T = run->n_passes;
   const size_t n_grad_all = (size_t)n_params * nv;
-  if ((rc = ensure(&ctx->d_adj_ck, ctx->adj_ck_cap, (size_t)std::max(grad ? T - 1 : 0, 1L) * 4 * np)) ||
-      (rc = ensure(&ctx->d_adj_grad, ctx->adj_grad_cap, std::max<size_t>(n_grad_all, 1))) ||
+  if ((rc = ensure(&ctx->d_adj_grad, ctx->adj_grad_cap, std::max<size_t>(n_grad_all, 1))) ||
       (rc = ensure(&ctx->d_adj_param, ctx->adj_param_cap, op_param.size())) ||
       (rc = ensure(&ctx->d_adj_dk, ctx->adj_dk_cap, op_dk.size())) ||
       (rc = ensure(&ctx->d_adj_dfo, ctx->adj_dfo_cap, op_dfield.size())) ||
       (rc = ensure(&ctx->d_adj_dfield, ctx->adj_dfield_cap, std::max<size_t>(dfield.size(), 1))))
     return rc;
+  /* Segments the reverse sweep inverts in one go (adj_reverse_kernel).  The
+   * error grows with a segment's own amplification squared.  Eight elements
+   * amplify by a few: on an unstable line that grows by 16 over eight and by
+   * 1e7 in all the gradient is within 1.2e-15 of the one from every element's
+   * recorded entry state.  At most T + nops states of 32 B per particle are
+   * kept, so segments are longer in runs of many passes, in each of which a
+   * beam within the coordinate limit can grow less.  Fewer where the memory
+   * does not hold them.  Kept states cost 2 % of the FODO ring's run of 8
+   * turns (1e5 particles, 38.1 -> 38.9 ms); a state per element 3 %. */
+  int every = std::max(nops, 1);
+  if (grad && nops > 0)
+    for (long segs = std::min<long>(1 + nops / T, (nops + 7) / 8);; segs /= 2) {
+      every = (int)((nops + segs - 1) / segs);
+      segs = (nops + every - 1) / every;
+      rc = ensure(&ctx->d_adj_ck, ctx->adj_ck_cap, std::max<size_t>((size_t)(T * segs - 1) * 4 * np, 1));
+      if (rc == TRK_OK)
+        break;
+      if (segs == 1)
+        return rc;
+      cudaGetLastError();
+    }
   CUDA_TRY(cudaMemcpyAsync(ctx->d_adj_dfo, op_dfield.data(), sizeof(int) * op_dfield.size(), cudaMemcpyHostToDevice,
                            ctx->stream));
   if (!dfield.empty())
@@ -2066,7 +2086,7 @@ static int adjoint_run(trk_context *ctx, const trk_lattice *const *lattices, int
   CUDA_TRY(cudaMemcpyAsync(ctx->d_adj_dk, op_dk.data(), sizeof(double) * op_dk.size(), cudaMemcpyHostToDevice,
                            ctx->stream));
 
-  /* forward, one pass per launch, the beam at the end of every pass but the last kept */
+  /* forward, at most 64 passes a launch */
   const long p0 = run->pass_offset;
   const long fresh = ctx->passes_done == 0 ? p0 : -1;
   if (fresh >= 0)
@@ -2079,19 +2099,21 @@ static int adjoint_run(trk_context *ctx, const trk_lattice *const *lattices, int
   ta.op_end = nops;
   const long *d_off = ensemble ? ctx->d_ens_offsets : nullptr;
   const int shape = trk_default_variant(true, c, ctx->np, ctx->sm_count);
-  for (long t = 0; t < T; t++) {
+  if (ensemble) {
+    ta.ens_offsets = d_off;
+    ta.ens_variants = nv;
+    ta.ens_ops = nops;
+  }
+  ta.rec = ctx->d_adj_ck;
+  ta.rec_every = every;
+  ta.rec_begin = p0;
+  for (long t = 0; t < T && nops > 0; t += 64) {
     ta.pass_begin = p0 + t;
-    ta.pass_end = p0 + t + 1;
-    if (nops > 0) {
-      if (ensemble)
-        trk_fast::launch_track_ensemble(ta, d_off, nv, nops, shape, trk_lean_flavor(c), np, ctx->sm_count * 256,
-                                        ctx->stream);
-      else
-        trk_fast::launch_track(ta, shape, trk_lean_flavor(c), np, ctx->sm_count * 256, ctx->stream);
-    }
-    for (int q = 0; q < 4 && grad && t < T - 1; q++)
-      CUDA_TRY(cudaMemcpyAsync(ctx->d_adj_ck + ((size_t)t * 4 + q) * np, ctx->d_cols + (size_t)q * ctx->cap,
-                               sizeof(double) * np, cudaMemcpyDeviceToDevice, ctx->stream));
+    ta.pass_end = p0 + std::min(t + 64, T);
+    if (grad)
+      trk_fast::launch_track_record(ta, shape, trk_lean_flavor(c), np, ctx->sm_count * 256, ctx->stream);
+    else
+      trk_fast::launch_track(ta, shape, trk_lean_flavor(c), np, ctx->sm_count * 256, ctx->stream);
   }
   CUDA_TRY(cudaGetLastError());
   ctx->passes_done += T;
@@ -2104,7 +2126,7 @@ static int adjoint_run(trk_context *ctx, const trk_lattice *const *lattices, int
   if (!grad)
     return TRK_OK;
 
-  /* reverse: every pass backwards in one launch, from the final beam and the checkpoints */
+  /* reverse: the whole run backwards in one launch, from the final beam and the segments' states */
   std::vector<double> coef(3 * (size_t)nv);
   for (int v = 0; v < nv; v++) {
     const double cnt = mom[4 * v + 3];
@@ -2127,12 +2149,8 @@ static int adjoint_run(trk_context *ctx, const trk_lattice *const *lattices, int
   g.op_dfield = ctx->d_adj_dfo;
   g.dfield = ctx->d_adj_dfield;
   g.n_ops = nops;
+  g.every = every;
   g.n_params = n_params;
-  if (ensemble) {
-    ta.ens_offsets = d_off;
-    ta.ens_variants = nv;
-    ta.ens_ops = nops;
-  }
   trk_fast::launch_adjoint_reverse(ta, g, ctx->stream);
   CUDA_TRY(cudaGetLastError());
   CUDA_TRY(cudaMemcpyAsync(grad, ctx->d_adj_grad, sizeof(double) * n_grad_all, cudaMemcpyDeviceToHost,

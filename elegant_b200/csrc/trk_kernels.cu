@@ -3127,11 +3127,29 @@ __device__ __forceinline__ bool after_element(const TrackArgs &a, const OpHead &
  * multipole or bend bodies); 2 as 1 plus combined-function bends, a flavour
  * of its own because their body, inlined into the loop, costs lattices
  * without them 3 % (register allocation of the whole loop) */
-template <int LEAN>
+template <int LEAN, bool REC>
 __device__ __forceinline__ bool track_particle(const TrackArgs &a, const trk_op *__restrict__ ops, Part &p, long i) {
+  /* REC: the next record (-1: the loaded beam) and the elements left before it */
+  long slot = -1;
+  int left = 0;
+  if (REC)
+    slot += (a.pass_begin - a.rec_begin) * ((a.op_end - a.op_begin + a.rec_every - 1) / a.rec_every);
   for (long pass = a.pass_begin; pass < a.pass_end; pass++) {
     const int var = (pass == a.fresh_pass) ? 0 : 1;
+    if (REC)
+      left = 0;
     for (int k = a.op_begin; k < a.op_end; k++) {
+      if (REC && left-- == 0) {
+        left = a.rec_every - 1;
+        if (slot >= 0) {
+          double *e = a.rec + (size_t)slot * 4 * a.n + i;
+          e[0] = p.x;
+          e[a.n] = p.xp;
+          e[2 * a.n] = p.y;
+          e[3 * a.n] = p.yp;
+        }
+        slot++;
+      }
       const trk_op *op = ops + k;
       const OpHead h = load_head(op, var);
       const trk_aperture *ap_in = h.ap_in >= 0 ? a.aps + h.ap_in : nullptr;
@@ -3232,7 +3250,7 @@ __device__ __forceinline__ int ens_variant(const long *__restrict__ offsets, int
 
 /* Kernel variants (block size, minimum resident blocks per SM) trade
  * registers against occupancy; trk_run.variant or the autotuner picks one. */
-template <int BLOCK, int MINB, int LEAN>
+template <int BLOCK, int MINB, int LEAN, bool REC = false>
 __global__ void __launch_bounds__(BLOCK, MINB) track_kernel(TrackArgs a) {
   const long stride = (long)gridDim.x * blockDim.x;
   const long n = a.live ? __ldg(a.live_n) : a.n;
@@ -3245,7 +3263,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) track_kernel(TrackArgs a) {
       ops += (long)ens_variant(a.ens_offsets, a.ens_variants, i) * a.ens_ops;
     Part p;
     load_part(a, i, p);
-    track_particle<LEAN>(a, ops, p, i);
+    track_particle<LEAN, REC>(a, ops, p, i);
     store_part(a, i, p);
   }
 }
@@ -3724,10 +3742,13 @@ __global__ void matrix_kernel(TrackArgs a, const double *__restrict__ m, int ord
  * Reverse mode through the fast build's element maps, in the momenta of the
  * merged bodies (divided by the total momentum).  The maps are inverted
  * exactly, substep by substep: a kick leaves the position it was taken at, a
- * drift the momenta (in a bend, a rotation).  So the sweep needs no recorded
- * states inside a pass: it starts from the beam at the end of the pass (the
- * next pass's checkpoint) and carries the particle and its adjoint (lambda of
- * x, x', y, y') back through the elements together.  One thread takes one
+ * drift the momenta (in a bend, a rotation).  The sweep starts from the final
+ * beam and carries the particle and its adjoint (lambda of x, x', y, y') back
+ * through the elements together.  A map that amplifies by G amplifies the
+ * rounding of its exit state by up to G on the way back, G^2 of the entry
+ * state, so the forward run keeps the entry state of every segment of a few
+ * elements (track_kernel's REC) and each segment starts from its exit's.  One
+ * thread takes one
  * particle through all passes of the run.  Parameter sensitivities of the
  * kick strengths are summed per warp and added to the gradient with one
  * atomic per warp and element.  delta has no adjoint: nothing on this path
@@ -3975,15 +3996,27 @@ __global__ void __launch_bounds__(128, 4) adj_reverse_kernel(TrackArgs a, AdjArg
     q.lx = fma(2 * q.x, c[2], c[0]);
     q.ly = fma(2 * q.y, c[2], c[1]);
   }
-  for (long t = g.n_passes - 1; t >= 0; t--) {
-    if (act && t < g.n_passes - 1) {
-      const double *e = g.ck + (size_t)t * 4 * n;
-      q.x = e[i];
-      q.px = e[n + i];
-      q.y = e[2 * n + i];
-      q.py = e[3 * n + i];
+  const int segs = (g.n_ops + g.every - 1) / g.every;
+  const long last = g.n_passes * segs - 1;
+  double ex = 0, exp_ = 0, ey = 0, eyp = 0;
+  for (long m = last; m >= 0; m--) {
+    /* the segment's exit state: the entry of the next (the last one's: the
+     * final beam), loaded a segment ahead */
+    if (m < last) {
+      q.x = ex;
+      q.px = exp_;
+      q.y = ey;
+      q.py = eyp;
     }
-    for (int k = g.n_ops - 1; k >= 0; k--) {
+    if (act && m > 0) {
+      const double *e = g.ck + (size_t)(m - 1) * 4 * n;
+      ex = e[i];
+      exp_ = e[n + i];
+      ey = e[2 * n + i];
+      eyp = e[3 * n + i];
+    }
+    const int k0 = (int)(m % segs) * g.every;
+    for (int k = min(k0 + g.every, g.n_ops) - 1; k >= k0; k--) {
       const trk_op *op = ops + k;
       double sk[2] = {0, 0};
       const int prm = __ldg(&g.op_param[k]);
@@ -4155,6 +4188,28 @@ void launch_track_ensemble(const TrackArgs &a, const long *offsets, int n_varian
   e.ens_variants = n_variants;
   e.ens_ops = ops_per_variant;
   launch_track(e, ensemble_variant_ok(variant) ? variant : 1, lean, n, max_blocks, st);
+}
+
+/* the forward run of a gradient: the shapes trk_default_variant picks for the lean flavours */
+void launch_track_record(const TrackArgs &a, int variant, int lean, long n, int max_blocks, cudaStream_t st) {
+#if TRK_FAST
+  const int g = (int)std::min<long>(std::max<long>((n + 127) / 128, 1), max_blocks);
+  if (lean == 2 && variant == 4)
+    track_kernel<128, 5, 2, true><<<g, 128, 0, st>>>(a);
+  else if (lean == 2)
+    track_kernel<128, 4, 2, true><<<g, 128, 0, st>>>(a);
+  else if (variant == 7)
+    track_kernel<128, 6, 1, true><<<g, 128, 0, st>>>(a);
+  else
+    track_kernel<128, 4, 1, true><<<g, 128, 0, st>>>(a);
+#else
+  (void)a;
+  (void)variant;
+  (void)lean;
+  (void)n;
+  (void)max_blocks;
+  (void)st;
+#endif
 }
 
 void launch_adjoint_reverse(const TrackArgs &a, const AdjArgs &g, cudaStream_t st) {

@@ -51,6 +51,11 @@ struct TrackArgs {
    * live[0 .. *live_n) (indices into the beam, ascending) instead of 0..n */
   const long *live;
   const long *live_n;
+  /* gradient runs: every rec_every-th element's entry x, xp, y, yp, four columns of n per record; pass rec_begin's
+   * first is the loaded beam and not kept */
+  double *rec;
+  int rec_every;
+  long rec_begin;
 };
 
 struct TimeStatsArgs {
@@ -114,7 +119,8 @@ struct WakeArgs {
 /* reverse-mode adjoint of the fast build's element maps (DRIF, EDRIFT,
  * single-order multipoles, CSBEND pure dipoles and K1/K2 expansions) */
 struct AdjArgs {
-  const double *ck;      /* beam at the end of pass t (t < n_passes - 1) at ck + t * 4 n: x, xp, y, yp columns */
+  const double *ck;      /* entry states of the segments after the first, in tracking order: x, xp, y, yp columns of n */
+  int every;             /* elements per segment; each pass starts one */
   const double *coef;    /* per variant: loss gradient coefficients (2 w mean(x)/N, 2 w mean(y)/N, 1/N) */
   double *grad;          /* gradient accumulators, one per parameter */
   const int *op_param;   /* parameter index of each op, -1 if none */
@@ -144,6 +150,8 @@ struct AdjArgs {
                     int elem, int grid, cudaStream_t st);                                                    \
   void launch_matrix(const TrackArgs &a, const double *m, int order, int grid, cudaStream_t st);             \
   int ensemble_variant_ok(int variant);                                                                      \
+  void launch_track_record(const TrackArgs &a, int variant, int lean, long n, int max_blocks,                \
+                           cudaStream_t st);                                                                 \
   void launch_adjoint_reverse(const TrackArgs &a, const AdjArgs &g, cudaStream_t st);                        \
   void launch_track_ensemble(const TrackArgs &a, const long *offsets, int n_variants, int ops_per_variant,   \
                              int variant, int lean, long n, int max_blocks, cudaStream_t st);               \

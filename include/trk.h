@@ -437,15 +437,15 @@ int trk_wake_noalloc(double *const *columns, int32_t *lost_pass, int32_t *lost_e
 /* Reverse-mode adjoint through the fused element chain (no counterpart in
  * the reference, which offers only finite differences through repeated
  * tracking).  Tracks the loaded beam n_passes passes (fast build), keeping
- * the beam at the start of every pass on the device, then sweeps back pass
- * by pass: each pass is recomputed from its checkpoint with every element's
- * entry state recorded, and the elements' hand-written adjoints carry
- * d(loss)/d(coordinates) backwards while the kick-strength sensitivities are
+ * the states the reverse sweep restarts from on the device (at most one per
+ * pass and element of one pass), then sweeps back: the elements' maps are
+ * inverted and their hand-written adjoints carry d(loss)/d(coordinates)
+ * backwards while the kick-strength sensitivities are
  * summed into the gradient.  Loss function over the surviving particles:
  *   loss = mean_i (x_i^2 + y_i^2) + w_c ((mean_i x_i)^2 + (mean_i y_i)^2)
  * (particles lost during the run are left out: loss events are not
- * differentiable).  Parameters: K1 of every KQUAD and K2 of every KSEXT, in
- * lattice order.  Elements allowed: DRIF, EDRIFT, single-order
+ * differentiable).  Parameters: K1 of every KQUAD, K2 of every KSEXT, K1 and
+ * K2 of every CSBEND, in lattice order.  Elements allowed: DRIF, EDRIFT, single-order
  * KQUAD/KSEXT/KOCT without tilt or misalignment, CSBEND (pure dipole, or a
  * K1/K2 field expansion) without misalignment or edge kick, MARK, MAXAMP.
  * grad may be NULL (loss only).  The device beam is left at its final state. */
@@ -462,7 +462,7 @@ int trk_adjoint_ensemble(trk_context *ctx, const trk_lattice *const *lattices, i
 /* The same loss function on the device beam as it is (for finite
  * differences against trk_adjoint). */
 int trk_objective(trk_context *ctx, double centroid_weight, double *loss);
-/* Number of gradient parameters (KQUAD K1 + KSEXT K2) of a lattice. */
+/* Number of gradient parameters (KQUAD K1, KSEXT K2, CSBEND K1 and K2) of a lattice. */
 int trk_adjoint_param_count(const trk_lattice *lattice);
 
 #ifdef __cplusplus

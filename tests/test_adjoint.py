@@ -7,7 +7,7 @@ gradient error <= 1e-6."""
 import numpy as np
 import pytest
 
-from elegant_b200 import Tracker, configs
+from elegant_b200 import Lattice, Tracker, configs
 from elegant_b200.adjoint import fd_step, get_parameters, make_autograd, parameter_list, set_parameters
 from oracle import pyoracle
 
@@ -222,3 +222,24 @@ def test_adjoint_ensemble_rejects_elements_of_any_variant(element, change, first
         trk.load(configs.c5_beam(100, seed=98))
         with pytest.raises(RuntimeError):
             trk.adjoint_ensemble(lats, [50, 50], 2, PC, W)
+
+
+@pytest.mark.parametrize("cells, passes", [(20, 1), (24, 1), (10, 2)])
+def test_adjoint_of_an_amplifying_line(cells, passes):
+    """An unstable line: the horizontal motion grows by 1e6 (24 cells: 1e7)
+    over the run.  The reverse sweep inverts the maps, which amplifies the
+    rounding of a segment's exit state by the square of the segment's own
+    growth, so no segment may span much of the line."""
+    lat = Lattice()
+    for _ in range(cells):
+        lat.add("KQUAD", "Q", L=0.3, K1=-1.2, N_KICKS=8)
+        lat.add("DRIF", "D", L=1.0)
+    rng = np.random.Generator(np.random.Philox(99))
+    beam = rng.normal(size=(1000, 7)) * [1e-8, 1e-8, 1e-8, 1e-8, 1e-3, 1e-3, 0]
+    beam[:, 6] = np.arange(1, 1001)
+    with Tracker(0) as trk:
+        trk.load(beam)
+        loss, grad = trk.adjoint(lat, passes, PC, W)
+        assert trk.count() == 1000 and loss > (1e5 * 1e-8) ** 2
+        fd = _gpu_fd(trk, lat, beam, passes, W)
+    assert _rel_err(grad, fd) < 1e-6, (grad, fd)
