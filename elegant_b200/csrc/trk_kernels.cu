@@ -2370,12 +2370,13 @@ __device__ __forceinline__ bool momentum_plain(double opd) {
 }
 
 /* true if every point of the box |x| <= xb, |y| <= yb passes check_aperture:
- * its elliptical test in products, with a margin above their roundings */
+ * its elliptical test in products, with a margin above their roundings, and
+ * with exponent 2 whatever the exponents, which are even and at least 2
+ * (trk_compile): |u|^m <= u^2 where |u| < 1, so a superellipse holds every
+ * point of its ellipse */
 __device__ __forceinline__ bool box_inside(double xb, double yb, const trk_aperture *__restrict__ ap) {
   const double xmax = __ldg(&ap->x_max), ymax = __ldg(&ap->y_max);
   if (__ldg(&ap->elliptical) && xmax > 0 && ymax > 0) {
-    if (__ldg(&ap->xexp) != 2 || __ldg(&ap->yexp) != 2)
-      return false;
     const double a2 = xmax * xmax, b2 = ymax * ymax;
     return fma(xb * xb, b2, yb * yb * a2) < a2 * b2 * (1 - 0x1p-40);
   }
