@@ -2361,6 +2361,12 @@ __device__ __forceinline__ double cos_m1(double z) {
 /* a double above every |v| whose high word is h */
 __device__ __forceinline__ double above(unsigned h) { return __hiloint2double((int)(h + 1), 0); }
 
+/* the bound on z of a multipole's entry slopes, whose first drift takes them as
+ * they are, from ss = 1 + x'^2 + y'^2: 0, or above every z's high word */
+__device__ __forceinline__ unsigned entry_z(double ss) {
+  return (unsigned)__double2hiint(ss) < 0x3ff00100u ? 0u : 0xffffffffu;
+}
+
 /* limits on |x|, |y| at the element's ends and 1 + delta > 0, by high word:
  * below 8 (the reference's limit is 10) and in (2^-31, 2^1000) */
 #define TRK_COORD_HI 0x40200000u
@@ -2403,7 +2409,7 @@ __device__ __forceinline__ bool mult1_merged(const double *__restrict__ d, int n
   double x = p.x, y = p.y, px = p.xp * r0, py = p.yp * r0;
   const double l0 = __ldg(&d[MD_DSH]), l1 = __ldg(&d[MD_DSH + 1]);
   const double ka = kick_over(__ldg(&d[MD_KQ]), opd, iopd), kb = kick_over(__ldg(&d[MD_KQ + 3]), opd, iopd);
-  unsigned zm = 0;
+  unsigned zm = entry_z(ss);
   double s = l0 * (ss * r0), v = 0; /* first drift: slopes xp, sqrt(1 + xp^2 + yp^2) */
   x = fma(p.xp, l0, x);
   y = fma(p.yp, l0, y);
@@ -2744,7 +2750,7 @@ __device__ __forceinline__ bool mult1_radiating(const trk_op *__restrict__ op, P
   const double r0 = rsqrt_fast(ss);
   double x = p.x, y = p.y, px = p.xp * r0, py = p.yp * r0;
   const double l0 = __ldg(&d[MD_DSH]), l1 = __ldg(&d[MD_DSH + 1]);
-  unsigned zm = 0, xm = hi_abs(x), ym = hi_abs(y);
+  unsigned zm = entry_z(ss), xm = hi_abs(x), ym = hi_abs(y);
   double s = l0 * (ss * r0), v = 0;
   x = fma(p.xp, l0, x);
   y = fma(p.yp, l0, y);

@@ -103,3 +103,17 @@ def test_superellipse_costs_what_an_ellipse_does(tracker, rad):
                 e[2]["SYNCH_RAD"] = rad
         ms[exponent] = min(gpu_run(tracker, lat, beam, 1, PC, fast=True)[4]["device_ms"] for _ in range(5))
     assert ms[4] < 2 * ms[2], ms
+
+
+def test_entry_slope_above_the_limit_is_a_loss(tracker):
+    """x' = 1.2 is a loss at the element's entry even where the kicks take
+    nearly all of it away: strength and position are solved for momenta below
+    1e-4 after each of the three kicks."""
+    lat = Lattice()
+    lat.add("KQUAD", "Q", L=0.1, K1=5604218.137052551, N_KICKS=4)
+    beam = np.zeros((2, 7))
+    beam[0, :2], beam[:, 6] = [-0.08107141710017259, 1.2], [1, 2]
+    nl, g, lp, le, _ = gpu_run(tracker, lat, beam, 1, PC, fast=True)
+    with pyoracle.modes(exact_sums=True, cr_math=True):
+        rows, nlo, _ = oracle_run(lat, beam, 1, PC)
+    assert compare(g, rows, nl, nlo)["same_survivors"] and nl == 1
