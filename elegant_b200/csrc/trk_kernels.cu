@@ -2336,6 +2336,7 @@ __device__ __forceinline__ bool op_cfbend_fast(const trk_op *__restrict__ op, Pa
  * integer maximum of high words (ALU pipe) and by the ends' positions: a
  * particle near any of them leaves the body unchanged and takes the checked one
  * (op_mult1_fast and so on), which locates the loss as the reference does.
+ * Slopes above the polynomials' range take the same bodies with roots (WIDE).
  * Bound by FP64 issue and by the length of the substep's chain (13 of its 17
  * operations).  Measured against the checked bodies alone, ms per turn: FODO
  * ring with RF and wake, 1e6 particles, 11.4 -> 7.5; achromat ring, 2e6, 250
@@ -2358,13 +2359,47 @@ __device__ __forceinline__ double cos_m1(double z) {
   return z * fma(z, fma(z, TRK_ECON3(1.0 / 16, a4), TRK_ECON2(1.0 / 8, a4)), TRK_ECON1(1.0 / 2, a4));
 }
 
+/* The same for any z < 1 where WIDE, the wide bodies' form for warps with a
+ * steep lane, by root and select: a branch around the root costs 10 % more.
+ * One cell of the FODO ring with sextupoles, 8e5 particles of 12 mrad: 0.28 ms,
+ * both bodies one after the other 0.41, the unmerged alone 0.26; of 10 urad
+ * 0.18. */
+template <bool WIDE> __device__ __forceinline__ double sec_m1_t(double z) {
+  const double v = sec_m1(z);
+  if (!WIDE)
+    return v;
+  const double u = rsqrt_fast(1 - z) - 1;
+  return (unsigned)__double2hiint(z) >= TRK_Z_HI ? u : v;
+}
+template <bool WIDE> __device__ __forceinline__ double cos_m1_t(double z) {
+  const double h = cos_m1(z);
+  if (!WIDE)
+    return h;
+  const double w = 1 - z, g = fma(-w, rsqrt_fast(w), 1.0);
+  return (unsigned)__double2hiint(z) >= TRK_Z_HI ? g : h;
+}
+/* the bound on z: 2^-12, WIDE 1/4, where slopes stay below their limit of 1 */
+template <bool WIDE> __device__ __forceinline__ bool z_accepted(unsigned zm) {
+  return zm < (WIDE ? 0x3fd00000u : TRK_Z_HI);
+}
+
 /* a double above every |v| whose high word is h */
 __device__ __forceinline__ double above(unsigned h) { return __hiloint2double((int)(h + 1), 0); }
 
 /* the bound on z of a multipole's entry slopes, whose first drift takes them as
  * they are, from ss = 1 + x'^2 + y'^2: 0, or above every z's high word */
-__device__ __forceinline__ unsigned entry_z(double ss) {
-  return (unsigned)__double2hiint(ss) < 0x3ff00100u ? 0u : 0xffffffffu;
+template <bool WIDE> __device__ __forceinline__ unsigned entry_z(double ss) {
+  return (unsigned)__double2hiint(ss) < (WIDE ? 0x3ff40000u : 0x3ff00100u) ? 0u : 0xffffffffu;
+}
+
+/* whether a lane of the warp enters with a slope at which the narrow body may
+ * end up above its bound (high word of the slope below which it does not).
+ * Such a warp takes the wide body at once.  Where both accept a particle they
+ * do the same operations, so its track does not depend on its neighbours. */
+#define TRK_STEEP_MULT 0x3f86a09eu /* 2^-6.5 in each plane: z = 2^-12 */
+#define TRK_STEEP_BEND 0x3f747ae1u /* 0.005: the bend's own swing adds up to 0.0085 (trk_compile) */
+__device__ __forceinline__ bool warp_steep(const Part &p, unsigned limit) {
+  return __any_sync(__activemask(), max(hi_abs(p.xp), hi_abs(p.yp)) >= limit);
 }
 
 /* limits on |x|, |y| at the element's ends and 1 + delta > 0, by high word:
@@ -2401,7 +2436,7 @@ __device__ __forceinline__ double kick_over(double k, double opd, double iopd) {
 /* OPK_MULT1; false: not taken, p unchanged.  Per kick: 2 to 8 operations of
  * the kick, 9 of the drift (13 and 15 in the unmerged body, with a reciprocal
  * square root). */
-template <int ORDER>
+template <int ORDER, bool WIDE>
 __device__ __forceinline__ bool mult1_merged(const double *__restrict__ d, int n_parts, Part &p) {
   const double opd = 1 + p.dp, iopd = rcp_fast(opd);
   const double ss = fma(p.yp, p.yp, fma(p.xp, p.xp, 1.0));
@@ -2409,7 +2444,7 @@ __device__ __forceinline__ bool mult1_merged(const double *__restrict__ d, int n
   double x = p.x, y = p.y, px = p.xp * r0, py = p.yp * r0;
   const double l0 = __ldg(&d[MD_DSH]), l1 = __ldg(&d[MD_DSH + 1]);
   const double ka = kick_over(__ldg(&d[MD_KQ]), opd, iopd), kb = kick_over(__ldg(&d[MD_KQ + 3]), opd, iopd);
-  unsigned zm = entry_z(ss);
+  unsigned zm = entry_z<WIDE>(ss);
   double s = l0 * (ss * r0), v = 0; /* first drift: slopes xp, sqrt(1 + xp^2 + yp^2) */
   x = fma(p.xp, l0, x);
   y = fma(p.yp, l0, y);
@@ -2431,7 +2466,7 @@ __device__ __forceinline__ bool mult1_merged(const double *__restrict__ d, int n
   {                                                                                                          \
     const double z = fma(py, py, px * px);                                                                   \
     zm = max(zm, (unsigned)__double2hiint(z));                                                               \
-    v = sec_m1(z);                                                                                           \
+    v = sec_m1_t<WIDE>(z);                                                                                   \
     const double l = fma((L), v, (L));                                                                       \
     x = fma(px, l, x);                                                                                       \
     y = fma(py, l, y);                                                                                       \
@@ -2448,7 +2483,7 @@ __device__ __forceinline__ bool mult1_merged(const double *__restrict__ d, int n
   }
 #undef TRK_KICK
 #undef TRK_DRIFT
-  if (!(zm < TRK_Z_HI && max(max(hi_abs(x), hi_abs(y)), max(hi_abs(p.x), hi_abs(p.y))) < TRK_COORD_HI &&
+  if (!(z_accepted<WIDE>(zm) && max(max(hi_abs(x), hi_abs(y)), max(hi_abs(p.x), hi_abs(p.y))) < TRK_COORD_HI &&
         momentum_plain(opd)))
     return false;
   p.x = x;
@@ -2466,6 +2501,7 @@ __device__ __forceinline__ bool mult1_merged(const double *__restrict__ d, int n
  * is px -= k R with R = rho0 + X, k = ds/(rho_actual rho0 (1 + delta)).  17
  * operations per kick and drift (20 with a root and a reciprocal in the
  * unmerged body). */
+template <bool WIDE>
 __device__ __forceinline__ bool dipole_merged(const double *__restrict__ d, int nSlices, Part &p) {
   const double rho0 = __ldg(&d[BD_RHO0]);
   const double opd = 1 + p.dp, iopd = rcp_fast(opd);
@@ -2480,11 +2516,11 @@ __device__ __forceinline__ bool dipole_merged(const double *__restrict__ d, int 
   double R = rho0 + X;
 #define TRK_DRIFT(SA, CA, OMC)                                                                               \
   {                                                                                                          \
-    const double z = fma(px, px, py2), h = cos_m1(z);                                                        \
+    const double z = fma(px, px, py2), h = cos_m1_t<WIDE>(z);                                                \
     const double m = fma(-(OMC), h, fma((SA), px, (OMC)));                                                   \
     px = fma(-(SA), h, fma((CA), px, (SA)));                                                                 \
     const double z1 = fma(px, px, py2);                                                                      \
-    v = sec_m1(z1);                                                                                          \
+    v = sec_m1_t<WIDE>(z1);                                                                                  \
     zm = max(zm, max((unsigned)__double2hiint(z), (unsigned)__double2hiint(z1)));                            \
     const double u = fma(R, v, R);                                                                           \
     X = fma(u, m, X);                                                                                        \
@@ -2510,7 +2546,7 @@ __device__ __forceinline__ bool dipole_merged(const double *__restrict__ d, int 
   }
 #undef TRK_DRIFT
   const double Y = fma(py, F, p.y);
-  if (!(zm < TRK_Z_HI && max(max(hi_abs(X), hi_abs(Y)), max(hi_abs(p.x), hi_abs(p.y))) < TRK_COORD_HI && momentum_plain(opd)))
+  if (!(z_accepted<WIDE>(zm) && max(max(hi_abs(X), hi_abs(Y)), max(hi_abs(p.x), hi_abs(p.y))) < TRK_COORD_HI && momentum_plain(opd)))
     return false;
   p.x = X;
   p.y = Y;
@@ -2522,7 +2558,7 @@ __device__ __forceinline__ bool dipole_merged(const double *__restrict__ d, int 
 
 /* OPK_CFBEND: the same with kicks that change py.  The field as in cf_fields;
  * LIN: K1 only, the midplane field linear in x and its slope constant. */
-template <bool LIN>
+template <bool LIN, bool WIDE>
 __device__ __forceinline__ bool cfbend_merged(const double *__restrict__ d, const double *__restrict__ fxy, int nSlices,
                                               Part &p) {
   const double rho0 = __ldg(&d[BD_RHO0]);
@@ -2537,16 +2573,16 @@ __device__ __forceinline__ bool cfbend_merged(const double *__restrict__ d, cons
 #define TRK_DRIFT(S, C, O)                                                                                   \
   {                                                                                                          \
     const double sa = __ldg(&dd[S]), co = __ldg(&dd[C]), omc = __ldg(&dd[O]);                                \
-    const double z = fma(px, px, py2), h = cos_m1(z);                                                        \
+    const double z = fma(px, px, py2), h = cos_m1_t<WIDE>(z);                                                \
     const double m = fma(-omc, h, fma(sa, px, omc));                                                         \
     px = fma(-sa, h, fma(co, px, sa));                                                                       \
     const double z1 = fma(px, px, py2);                                                                      \
-    v = sec_m1(z1);                                                                                          \
+    v = sec_m1_t<WIDE>(z1);                                                                                  \
     zm = max(zm, max((unsigned)__double2hiint(z), (unsigned)__double2hiint(z1)));                            \
     const double u = fma(R, v, R), us = u * sa;                                                              \
     X = fma(u, m, X);                                                                                        \
     Y = fma(py, us, Y);                                                                                      \
-    dist += us;                                                                                              \
+    dist = fma(u, sa, dist);                                                                                 \
     R = rho0 + X;                                                                                            \
   }
 #define TRK_KICK(K)                                                                                          \
@@ -2591,7 +2627,7 @@ __device__ __forceinline__ bool cfbend_merged(const double *__restrict__ d, cons
 #undef TRK_KICK
 #undef TRK_DRIFT
 #undef CF_T
-  if (!(zm < TRK_Z_HI && max(max(hi_abs(X), hi_abs(Y)), max(hi_abs(p.x), hi_abs(p.y))) < TRK_COORD_HI &&
+  if (!(z_accepted<WIDE>(zm) && max(max(hi_abs(X), hi_abs(Y)), max(hi_abs(p.x), hi_abs(p.y))) < TRK_COORD_HI &&
         momentum_plain(opd)))
     return false;
   p.x = X;
@@ -2602,23 +2638,34 @@ __device__ __forceinline__ bool cfbend_merged(const double *__restrict__ d, cons
   return true;
 }
 
-/* The checked bodies out of line for the particles the merged ones leave,
+/* The other bodies out of line, for the particles the narrow ones leave,
  * passed and returned by value (a reference would pin the caller's
- * coordinates in local memory).  All elements inside an aperture come here:
+ * coordinates in local memory): the wide merged body, and the checked one for
+ * what is near a loss.  All elements inside an aperture take the checked one:
  * particles near the dynamic aperture move chaotically, and any other order
  * of rounding changes their tracks by up to 1e-4 of the beam after 32 turns,
  * so aperture studies keep the unmerged arithmetic.  What they do not need is
  * the test in every slice, with its divisions: the body runs without it and
  * the box around the slice boundaries is tested in products; only a particle
  * whose box is not clear of the aperture is taken through the tests. */
-__device__ __noinline__ PartLoss mult1_checked(const trk_op *__restrict__ op, Part p, double Po, double z_start,
-                                               const trk_aperture *ap) {
+template <int ORDER>
+__device__ __forceinline__ bool mult1_wide(const trk_op *__restrict__ op, Part &p) {
+  return mult1_merged<ORDER, true>(op->d, __ldg(&op->i[0]), p);
+}
+
+__device__ __noinline__ PartLoss mult1_other(const trk_op *__restrict__ op, Part p, double Po, double z_start,
+                                             const trk_aperture *ap) {
   PartLoss r;
+  r.p = p;
+  r.lost = 0;
   if (ap) {
     unsigned box[2] = {0, 0};
-    r.p = p;
     r.lost = !op_mult1_fast(op, r.p, Po, z_start, nullptr, box);
     if (!r.lost && box_inside(above(box[0]), above(box[1]), ap))
+      return r;
+  } else {
+    const int order = __ldg(&op->i[4]) & 0xff;
+    if (order == 1 ? mult1_wide<1>(op, r.p) : order == 2 ? mult1_wide<2>(op, r.p) : mult1_wide<3>(op, r.p))
       return r;
   }
   r.lost = !op_mult1_fast(op, p, Po, z_start, ap);
@@ -2626,31 +2673,45 @@ __device__ __noinline__ PartLoss mult1_checked(const trk_op *__restrict__ op, Pa
   return r;
 }
 
-__device__ __noinline__ PartLoss dipole_checked(const trk_op *__restrict__ op, Part p, double Po, double z_start,
-                                                const trk_aperture *ap) {
+__device__ __noinline__ PartLoss dipole_other(const trk_op *__restrict__ op, Part p, double Po, double z_start,
+                                              const trk_aperture *ap) {
   PartLoss r;
+  r.p = p;
+  r.lost = 0;
   if (ap) {
     unsigned box[2] = {0, 0};
-    r.p = p;
     r.lost = !op_dipole_fast(op, r.p, Po, z_start, nullptr, box);
     if (!r.lost && box_inside(above(box[0]), above(box[1]), ap))
       return r;
-  }
+  } else if ((__ldg(&op->i[7]) & BF_MERGED) && dipole_merged<true>(op->d, __ldg(&op->i[0]), r.p))
+    return r;
   r.lost = !op_dipole_fast(op, p, Po, z_start, ap);
   r.p = p;
   return r;
 }
 
-__device__ __noinline__ PartLoss cfbend_checked(const trk_op *__restrict__ op, Part p, double Po, double z_start,
-                                                const trk_aperture *ap, const double *__restrict__ field) {
+/* OPK_CFBEND by the merged body its field asks for */
+template <bool WIDE>
+__device__ __forceinline__ bool cfbend_any(const trk_op *__restrict__ op, const double *__restrict__ field, int flags,
+                                           Part &p) {
+  const double *fxy = field + __ldg(&op->i[4]);
+  return (flags & BF_LINEAR) ? cfbend_merged<true, WIDE>(op->d, fxy, __ldg(&op->i[0]), p)
+                             : cfbend_merged<false, WIDE>(op->d, fxy, __ldg(&op->i[0]), p);
+}
+
+__device__ __noinline__ PartLoss cfbend_other(const trk_op *__restrict__ op, Part p, double Po, double z_start,
+                                              const trk_aperture *ap, const double *__restrict__ field) {
   PartLoss r;
+  r.p = p;
+  r.lost = 0;
+  const int flags = __ldg(&op->i[7]);
   if (ap) {
     unsigned box[2] = {0, 0};
-    r.p = p;
     r.lost = !op_cfbend_fast(op, r.p, Po, z_start, nullptr, field, box);
     if (!r.lost && box_inside(above(box[0]), above(box[1]), ap))
       return r;
-  }
+  } else if ((flags & BF_MERGED) && cfbend_any<true>(op, field, flags, r.p))
+    return r;
   r.lost = !op_cfbend_fast(op, p, Po, z_start, ap, field);
   r.p = p;
   return r;
@@ -2658,28 +2719,29 @@ __device__ __noinline__ PartLoss cfbend_checked(const trk_op *__restrict__ op, P
 
 __device__ __forceinline__ bool op_mult1(const trk_op *__restrict__ op, Part &p, double Po, double z_start,
                                          const trk_aperture *ap) {
-  const int n_parts = __ldg(&op->i[0]), order = __ldg(&op->i[4]) & 0xff;
-  bool done = false;
-  if (ap)
-    ;
-  else if (order == 1)
-    done = mult1_merged<1>(op->d, n_parts, p);
-  else if (order == 2)
-    done = mult1_merged<2>(op->d, n_parts, p);
-  else
-    done = mult1_merged<3>(op->d, n_parts, p);
-  if (done)
-    return true;
-  const PartLoss r = mult1_checked(op, p, Po, z_start, ap);
+  if (!ap && !warp_steep(p, TRK_STEEP_MULT)) {
+    const int n_parts = __ldg(&op->i[0]), order = __ldg(&op->i[4]) & 0xff;
+    bool done;
+    if (order == 1)
+      done = mult1_merged<1, false>(op->d, n_parts, p);
+    else if (order == 2)
+      done = mult1_merged<2, false>(op->d, n_parts, p);
+    else
+      done = mult1_merged<3, false>(op->d, n_parts, p);
+    if (done)
+      return true;
+  }
+  const PartLoss r = mult1_other(op, p, Po, z_start, ap);
   p = r.p;
   return !r.lost;
 }
 
 __device__ __forceinline__ bool op_dipole(const trk_op *__restrict__ op, Part &p, double Po, double z_start,
                                           const trk_aperture *ap) {
-  if (!ap && (__ldg(&op->i[7]) & BF_MERGED) && dipole_merged(op->d, __ldg(&op->i[0]), p))
+  if (!ap && (__ldg(&op->i[7]) & BF_MERGED) && !warp_steep(p, TRK_STEEP_BEND) &&
+      dipole_merged<false>(op->d, __ldg(&op->i[0]), p))
     return true;
-  const PartLoss r = dipole_checked(op, p, Po, z_start, ap);
+  const PartLoss r = dipole_other(op, p, Po, z_start, ap);
   p = r.p;
   return !r.lost;
 }
@@ -2687,13 +2749,9 @@ __device__ __forceinline__ bool op_dipole(const trk_op *__restrict__ op, Part &p
 __device__ __forceinline__ bool op_cfbend(const trk_op *__restrict__ op, Part &p, double Po, double z_start,
                                           const trk_aperture *ap, const double *__restrict__ field) {
   const int flags = __ldg(&op->i[7]);
-  if (!ap && (flags & BF_MERGED)) {
-    const double *fxy = field + __ldg(&op->i[4]);
-    if ((flags & BF_LINEAR) ? cfbend_merged<true>(op->d, fxy, __ldg(&op->i[0]), p)
-                            : cfbend_merged<false>(op->d, fxy, __ldg(&op->i[0]), p))
-      return true;
-  }
-  const PartLoss r = cfbend_checked(op, p, Po, z_start, ap, field);
+  if (!ap && (flags & BF_MERGED) && !warp_steep(p, TRK_STEEP_BEND) && cfbend_any<false>(op, field, flags, p))
+    return true;
+  const PartLoss r = cfbend_other(op, p, Po, z_start, ap, field);
   p = r.p;
   return !r.lost;
 }
@@ -2750,7 +2808,7 @@ __device__ __forceinline__ bool mult1_radiating(const trk_op *__restrict__ op, P
   const double r0 = rsqrt_fast(ss);
   double x = p.x, y = p.y, px = p.xp * r0, py = p.yp * r0;
   const double l0 = __ldg(&d[MD_DSH]), l1 = __ldg(&d[MD_DSH + 1]);
-  unsigned zm = entry_z(ss), xm = hi_abs(x), ym = hi_abs(y);
+  unsigned zm = entry_z<false>(ss), xm = hi_abs(x), ym = hi_abs(y);
   double s = l0 * (ss * r0), v = 0;
   x = fma(p.xp, l0, x);
   y = fma(p.yp, l0, y);
