@@ -2791,8 +2791,9 @@ __device__ __forceinline__ double rcp_update(double opd, double iopd) {
 /* path length scaled to the new velocity: beta(P1) s / beta(P0) */
 __device__ __forceinline__ double beta_of(double p) { return p / sqrt(sqr(p) + 1); }
 
-template <int ORDER>
-__device__ __forceinline__ bool mult1_radiating(const trk_op *__restrict__ op, Part &p, double Po,
+/* 1: taken; 0: too steep for the narrow form; -1: the general body's (p unchanged) */
+template <int ORDER, bool WIDE>
+__device__ __forceinline__ int mult1_radiating(const trk_op *__restrict__ op, Part &p, double Po,
                                                 const trk_aperture *__restrict__ ap, const IsrKey &key) {
   const double *d = op->d;
   const int n_parts = __ldg(&op->i[0]), flags = __ldg(&op->i[6]);
@@ -2803,12 +2804,12 @@ __device__ __forceinline__ bool mult1_radiating(const trk_op *__restrict__ op, P
   const double field = __ldg(&d[MD_KQ]) / (__ldg(&d[MD_KFRAC]) * len), field2 = field * field;
   double D = p.dp, opd = 1 + D, iopd = rcp_fast(opd);
   if (!momentum_plain(opd))
-    return false;
+    return -1;
   const double ss = fma(p.yp, p.yp, fma(p.xp, p.xp, 1.0));
   const double r0 = rsqrt_fast(ss);
   double x = p.x, y = p.y, px = p.xp * r0, py = p.yp * r0;
   const double l0 = __ldg(&d[MD_DSH]), l1 = __ldg(&d[MD_DSH + 1]);
-  unsigned zm = entry_z<false>(ss), xm = hi_abs(x), ym = hi_abs(y);
+  unsigned zm = entry_z<WIDE>(ss), xm = hi_abs(x), ym = hi_abs(y);
   double s = l0 * (ss * r0), v = 0;
   x = fma(p.xp, l0, x);
   y = fma(p.yp, l0, y);
@@ -2835,13 +2836,13 @@ __device__ __forceinline__ bool mult1_radiating(const trk_op *__restrict__ op, P
       py = fma(k, fx, py);
       const double z = fma(py, py, px * px);
       zm = max(zm, (unsigned)__double2hiint(z));
-      v = sec_m1(z);
+      v = sec_m1_t<WIDE>(z);
       const double F2 = field2 * fma(fx, fx, fy * fy);
-      double loss = rad * __ldg(&d[MD_KFRAC + j]) * F2 * (1 + v);
+      double loss = rad * __ldg(&d[MD_KFRAC + j]) * F2 * __dadd_rn(1.0, v);
       if (isr) {
         const double F = sqrt_fast(F2);
         const double g = isr_deviate(key.seed, key.id, key.pass, key.elem, (unsigned)(i * 8 + j), key.limit);
-        loss = fma(isr_c * F * sqrt_fast(F * (1 + v)), g, loss);
+        loss = fma(isr_c * F * sqrt_fast(F * __dadd_rn(1.0, v)), g, loss);
       }
       D = fma(-(opd * opd), loss, D);
       opd = 1 + D;
@@ -2854,10 +2855,12 @@ __device__ __forceinline__ bool mult1_radiating(const trk_op *__restrict__ op, P
   }
   xm = max(xm, hi_abs(x));
   ym = max(ym, hi_abs(y));
-  if (!(zm < TRK_Z_HI && max(xm, ym) < TRK_COORD_HI && momentum_plain(opd) && fabs(D - p.dp) < 1e-4 * opd))
-    return false;
+  if (!z_accepted<WIDE>(zm))
+    return 0;
+  if (!(max(xm, ym) < TRK_COORD_HI && momentum_plain(opd) && fabs(D - p.dp) < 1e-4 * opd))
+    return -1;
   if (ap && !box_inside(above(xm), above(ym), ap))
-    return false;
+    return -1;
   p.x = x;
   p.y = y;
   p.xp = fma(px, v, px);
@@ -2868,10 +2871,11 @@ __device__ __forceinline__ bool mult1_radiating(const trk_op *__restrict__ op, P
   } else
     p.s += s;
   p.dp = D;
-  return true;
+  return 1;
 }
 
-__device__ __forceinline__ bool dipole_radiating(const trk_op *__restrict__ op, Part &p, double Po,
+template <bool WIDE>
+__device__ __forceinline__ int dipole_radiating(const trk_op *__restrict__ op, Part &p, double Po,
                                                  const trk_aperture *__restrict__ ap, const IsrKey &key) {
   const double *d = op->d;
   const int nSlices = __ldg(&op->i[0]), flags = __ldg(&op->i[7]);
@@ -2880,7 +2884,7 @@ __device__ __forceinline__ bool dipole_radiating(const trk_op *__restrict__ op, 
   const double isr_c = isr ? __ldg(&d[BD_ISR]) * sqrt_fast(__ldg(&d[BD_SLICE]) * (1.0 / 3)) : 0;
   double D = p.dp, opd = 1 + D, iopd = rcp_fast(opd);
   if (!momentum_plain(opd))
-    return false;
+    return -1;
   const double r0 = rsqrt_fast(fma(p.yp, p.yp, fma(p.xp, p.xp, 1.0)));
   const double py = p.yp * r0, py2 = py * py;
   double px = p.xp * r0, X = p.x, F = 0, v = 0;
@@ -2896,9 +2900,9 @@ __device__ __forceinline__ bool dipole_radiating(const trk_op *__restrict__ op, 
       const double ca = __ldg(&d[BD_C2]), c = j == 1 ? fma(-2.0, ca, __ldg(&d[BD_KT])) : ca;
       px = fma(-(c * iopd), R, px);
     }
-    const double z = fma(px, px, py2), h = cos_m1(z);
+    const double z = fma(px, px, py2), h = cos_m1_t<WIDE>(z);
     if (k >= 0) {
-      const double hs = (R * rhoinv) * (1 + sec_m1(z));
+      const double hs = (R * rhoinv) * __dadd_rn(1.0, sec_m1_t<WIDE>(z));
       double loss = rad * __ldg(&d[BD_DS + j]) * hs;
       if (isr) {
         const double g =
@@ -2916,7 +2920,7 @@ __device__ __forceinline__ bool dipole_radiating(const trk_op *__restrict__ op, 
     const double m = fma(-omc, h, fma(sa, px, omc));
     px = fma(-sa, h, fma(ca, px, sa));
     const double z1 = fma(px, px, py2);
-    v = sec_m1(z1);
+    v = sec_m1_t<WIDE>(z1);
     zm = max(zm, max((unsigned)__double2hiint(z), (unsigned)__double2hiint(z1)));
     const double u = fma(R, v, R);
     X = fma(u, m, X);
@@ -2925,9 +2929,10 @@ __device__ __forceinline__ bool dipole_radiating(const trk_op *__restrict__ op, 
     xm = max(xm, hi_abs(X));
   }
   const double Y = fma(py, F, p.y);
-  if (!(zm < TRK_Z_HI && max(xm, max(hi_abs(p.y), hi_abs(Y))) < TRK_COORD_HI && momentum_plain(opd) &&
-        fabs(D - p.dp) < 1e-4 * opd))
-    return false;
+  if (!z_accepted<WIDE>(zm))
+    return 0;
+  if (!(max(xm, max(hi_abs(p.y), hi_abs(Y))) < TRK_COORD_HI && momentum_plain(opd) && fabs(D - p.dp) < 1e-4 * opd))
+    return -1;
   if (ap) {
     const double xb = above(xm);
     /* a slice boundary lies on a chord between two of these points, at most
@@ -2935,7 +2940,7 @@ __device__ __forceinline__ bool dipole_radiating(const trk_op *__restrict__ op, 
      * from slice to slice, so Y stays between its ends */
     if (!(xb < 0.125 * fabs(rho0)) || !box_inside(fma(2 * fabs(rho0), __ldg(&d[BD_OMC2]), xb),
                                                   above(max(hi_abs(p.y), hi_abs(Y))), ap))
-      return false;
+      return -1;
   }
   const double p0 = Po * (1 + p.dp), p1 = Po * opd;
   p.s = p1 / sqrt(sqr(p1) + 1) * p.s / (p0 / sqrt(sqr(p0) + 1)) + F;
@@ -2944,26 +2949,32 @@ __device__ __forceinline__ bool dipole_radiating(const trk_op *__restrict__ op, 
   p.xp = fma(px, v, px);
   p.yp = fma(py, v, py);
   p.dp = D;
-  return true;
+  return 1;
 }
 
 /* The general kernel calls the special bodies out of line: inlined beside the
  * general ones they took registers from both (radiating ring 5 % slower).
  * lost < 0: not taken. */
+template <bool WIDE>
+__device__ __forceinline__ int radiating_body(const trk_op *__restrict__ op, Part &p, double Po,
+                                               const trk_aperture *ap, const IsrKey &key) {
+  if (__ldg(&op->kind) == OPK_BEND)
+    return dipole_radiating<WIDE>(op, p, Po, ap, key);
+  const int order = __ldg(&op->i[4]) & 0xff;
+  return order == 1   ? mult1_radiating<1, WIDE>(op, p, Po, ap, key)
+         : order == 2 ? mult1_radiating<2, WIDE>(op, p, Po, ap, key)
+                      : mult1_radiating<3, WIDE>(op, p, Po, ap, key);
+}
+
 __device__ __noinline__ PartLoss radiating_call(const trk_op *__restrict__ op, Part p, double Po,
                                                 const trk_aperture *ap, IsrKey key) {
   PartLoss r;
   r.p = p;
-  bool done;
-  if (__ldg(&op->kind) == OPK_BEND)
-    done = dipole_radiating(op, r.p, Po, ap, key);
-  else {
-    const int order = __ldg(&op->i[4]) & 0xff;
-    done = order == 1   ? mult1_radiating<1>(op, r.p, Po, ap, key)
-           : order == 2 ? mult1_radiating<2>(op, r.p, Po, ap, key)
-                        : mult1_radiating<3>(op, r.p, Po, ap, key);
-  }
-  r.lost = done ? 0 : -1;
+  const bool steep = warp_steep(p, __ldg(&op->kind) == OPK_BEND ? TRK_STEEP_BEND : TRK_STEEP_MULT);
+  int done = steep ? 0 : radiating_body<false>(op, r.p, Po, ap, key);
+  if (done == 0)
+    done = radiating_body<true>(op, r.p, Po, ap, key);
+  r.lost = done == 1 ? 0 : -1;
   return r;
 }
 

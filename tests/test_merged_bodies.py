@@ -126,11 +126,14 @@ def _line_with_steep_lanes():
     return lat
 
 
-@pytest.mark.parametrize("variant", [-1, 4, 7])
-def test_tracks_do_not_depend_on_steep_neighbours(tracker, variant):
+@pytest.mark.parametrize("variant, rad", [(-1, 0.0), (4, 0.0), (7, 0.0), (-1, 1.0)])
+def test_tracks_do_not_depend_on_steep_neighbours(tracker, variant, rad):
     """A warp with a steep lane takes the bodies that hold for steep slopes;
     its other lanes keep every bit."""
     lat = _line_with_steep_lanes()
+    for e in lat.elements:
+        if e[0] in ("KQUAD", "KSEXT", "CSBEND"):
+            e[2]["SYNCH_RAD"], e[2]["ISR"] = rad, rad
     beam = configs.c5_beam(3000, seed=8)
     _, alone, _, _, _ = gpu_run(tracker, lat, beam, 2, PC, fast=True, variant=variant)
     mixed = beam.copy()
@@ -141,11 +144,16 @@ def test_tracks_do_not_depend_on_steep_neighbours(tracker, variant):
     assert np.array_equal(g[np.argsort(g[:, 6])][same], alone[np.argsort(alone[:, 6])][same])
 
 
-def test_steep_beam_takes_one_body(tracker):
+@pytest.mark.parametrize("rad", [0.0, 1.0])
+def test_steep_beam_takes_one_body(tracker, rad):
     """A divergent beam (12 mrad) once ran the merged and the unmerged body of
-    every element, 2.3 times a narrow beam's time; the wide bodies take 1.6."""
+    every element, 2.3 (radiating: 3.8) times a narrow beam's time; the wide
+    bodies take 1.6 (1.3)."""
     ms = {}
     lat = configs.c2_lattice(cells=1, with_rf=False, with_wake=False)
+    for e in lat.elements:
+        if e[0] in ("KQUAD", "KSEXT", "CSBEND"):
+            e[2]["SYNCH_RAD"], e[2]["ISR"] = rad, rad
     for slope in (0.0, 0.012):
         beam = configs.gaussian_beam(400000, seed=3)
         beam[:, 1], beam[:, 3] = beam[:, 1] * slope / 10e-6, beam[:, 3] * slope / 10e-6
