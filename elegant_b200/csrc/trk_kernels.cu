@@ -2443,7 +2443,14 @@ __device__ __forceinline__ bool mult1_merged(const double *__restrict__ d, int n
   const double r0 = rsqrt_fast(ss);
   double x = p.x, y = p.y, px = p.xp * r0, py = p.yp * r0;
   const double l0 = __ldg(&d[MD_DSH]), l1 = __ldg(&d[MD_DSH + 1]);
-  const double ka = kick_over(__ldg(&d[MD_KQ]), opd, iopd), kb = kick_over(__ldg(&d[MD_KQ + 3]), opd, iopd);
+  /* The three kicks of a slice add up to its whole kick, rounded once (the two
+   * differences are exact): a kick's rounding is the same in every element of a
+   * kind, so it moves the tune, and three kicks rounded apart left twice the
+   * error in y and y' on the FODO ring.  Costs 1 % at 1e4 particles, nothing
+   * that shows at 1e6. */
+  const double k0 = __ldg(&d[MD_KQ]), k1 = __ldg(&d[MD_KQ + 3]);
+  const double ka = __dmul_rn(k0, iopd), kb = __dmul_rn(k1, iopd);
+  const double kc = (kick_over(fma(2.0, k0, k1), opd, iopd) - ka) - kb;
   unsigned zm = entry_z<WIDE>(ss);
   double s = l0 * (ss * r0), v = 0; /* first drift: slopes xp, sqrt(1 + xp^2 + yp^2) */
   x = fma(p.xp, l0, x);
@@ -2478,7 +2485,7 @@ __device__ __forceinline__ bool mult1_merged(const double *__restrict__ d, int n
     TRK_DRIFT(l1)
     TRK_KICK(kb)
     TRK_DRIFT(l1)
-    TRK_KICK(ka)
+    TRK_KICK(kc)
     TRK_DRIFT(le)
   }
 #undef TRK_KICK
