@@ -1118,7 +1118,7 @@ int trk_track(trk_context *ctx, const trk_lattice *lattice, const trk_run *run, 
   if (variant < 0 || variant >= TRK_N_VARIANTS)
     variant = ctx->tuned_variant;
   if (variant < 0)
-    variant = trk_default_variant(fast, c, ctx->np, ctx->sm_count);
+    variant = trk_default_variant(c, ctx->np, ctx->sm_count);
   CUDA_TRY(cudaEventRecord(ctx->ev0, ctx->stream));
   if (ctx->np > 0 && run->n_passes > 0 && fresh >= 0) {
     screen_kernel<<<(int)((ctx->np + 255) / 256), 256, 0, ctx->stream>>>(
@@ -1333,7 +1333,7 @@ int trk_track_element(trk_context *ctx, const trk_lattice *lattice, int element,
   const bool fast = run->fast_math != 0;
   int variant = run->variant;
   if (variant < 0 || variant >= TRK_N_VARIANTS)
-    variant = trk_default_variant(fast, c, ctx->np, ctx->sm_count);
+    variant = trk_default_variant(c, ctx->np, ctx->sm_count);
   ctx->last_launches = 0;
   if (k >= 0 && (ctx->np > 0 || ctx->comm)) {
     const trk_op &op = c.ops[k];
@@ -2098,7 +2098,7 @@ static int adjoint_run(trk_context *ctx, const trk_lattice *const *lattices, int
   ta.op_begin = 0;
   ta.op_end = nops;
   const long *d_off = ensemble ? ctx->d_ens_offsets : nullptr;
-  const int shape = trk_default_variant(true, c, ctx->np, ctx->sm_count);
+  const int shape = trk_default_variant(c, ctx->np, ctx->sm_count);
   if (ensemble) {
     ta.ens_offsets = d_off;
     ta.ens_variants = nv;

@@ -45,20 +45,16 @@ inline int trk_lean_flavor(const CompiledLattice &c) { return c.lean ? (c.has_cf
  * particles on sms SMs (ms per turn on B200, this rule's choice first):
  *  - up to 4 warps a scheduler, 512 particles an SM, (128 threads, 4 blocks/SM):
  *    more blocks would not be resident anyway, and 128 registers spill nothing
- *    (FODO ring, 1e4 particles: 0.39 against 0.43 at (128, 6); parity build,
- *    30,011 particles with sextupoles: 3.2 against 3.8);
+ *    (FODO ring, 1e4 particles: 0.36 against 0.41 at (128, 6); parity build,
+ *    30,011 particles with sextupoles: 3.3 against 3.8);
  *  - lean lattices without combined-function bends, (128, 6): FODO ring with RF
- *    and wake, 1e6 particles, parity 57.7 against 61.1 at (128, 4), fast 7.65
- *    against 7.97 (before the merged bodies left the aperture to the checked ones);
- *  - fast build with combined-function bends, (128, 5), which their body needs
- *    not to spill: achromat ring, 1e6 particles, 79.6 against 81.3 at (128, 6);
- *  - (128, 4) otherwise. */
-inline int trk_default_variant(bool fast, const CompiledLattice &c, long np, int sms) {
-  if (np <= 512L * sms)
-    return 1;
-  if (c.lean && (fast || !c.has_cfbend))
-    return fast && c.has_cfbend ? 4 : 7;
-  return 1;
+ *    and wake, 1e6 particles, parity 57.7 against 61.3 at (128, 4), fast 7.5
+ *    against 7.8;
+ *  - (128, 4) otherwise, with combined-function bends because their body spills
+ *    at fewer registers: achromat ring, 2e6 particles, 147.1 against 148.5 at
+ *    (128, 5) and (128, 6); 3e5 particles 23.9 against 25.2 and 24.7. */
+inline int trk_default_variant(const CompiledLattice &c, long np, int sms) {
+  return np > 512L * sms && c.lean && !c.has_cfbend ? 7 : 1;
 }
 
 int trk_compile(const trk_lattice *l, double Po, CompiledLattice &out);

@@ -4277,9 +4277,7 @@ void launch_track_ensemble(const TrackArgs &a, const long *offsets, int n_varian
 void launch_track_record(const TrackArgs &a, int variant, int lean, long n, int max_blocks, cudaStream_t st) {
 #if TRK_FAST
   const int g = (int)std::min<long>(std::max<long>((n + 127) / 128, 1), max_blocks);
-  if (lean == 2 && variant == 4)
-    track_kernel<128, 5, 2, true><<<g, 128, 0, st>>>(a);
-  else if (lean == 2)
+  if (lean == 2)
     track_kernel<128, 4, 2, true><<<g, 128, 0, st>>>(a);
   else if (variant == 7)
     track_kernel<128, 6, 1, true><<<g, 128, 0, st>>>(a);
