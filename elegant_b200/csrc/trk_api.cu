@@ -1976,7 +1976,8 @@ static int adjoint_run(trk_context *ctx, const trk_lattice *const *lattices, int
   std::vector<int> op_dfield(std::max(nops, 1), -1);
   std::vector<double> dfield;
   std::vector<const trk_elem *> dfield_elem; /* the bend each table was formed for */
-  /* the kinds depend on parameter values, so every variant's records are looked at */
+  /* the kinds depend on parameter values, so every variant's records are looked
+   * at (the limits on slices are the interface's; the sweep takes any number) */
   for (int k = 0; k < nops * nv; k++) {
     const trk_op &op = c.ops[k];
     switch (op.kind) {

@@ -1024,8 +1024,8 @@ int trk_compile(const trk_lattice *l, double Po, CompiledLattice &out) {
     }
     if (rc != TRK_OK)
       return rc;
-    /* kinds with a specialized fast-build body (the parity build runs the
-     * general body for them) */
+    /* kinds with a body of their own (combined-function bends in the fast build
+     * only: the parity build runs the general body for them) */
     if (op.kind == OPK_MULT) {
       const int f = op.i[6];
       const int o = op.i[4] & 0xff;

@@ -762,8 +762,10 @@ __device__ __forceinline__ double tiny_sum(double lead, double c, unsigned long 
  *    corrections (by f, rho0, rho_actual, 1 + delta from double-double
  *    reciprocals formed once, by the two cosines from rcp_below1), and the
  *    range that all of this needs in two integer maxima.  If anything fails,
- *    the substep is redone by dipole_drift_checked, for one warp in 70 on the
- *    FODO ring's bends;
+ *    the substep is redone by dipole_drift_checked, for one warp in 77 on the
+ *    FODO ring's bends (counted on the host).  Bends of coarse slices and steep
+ *    beams redo most substeps: up to 10 % slower than the branching form alone,
+ *    where tests for it beforehand cost every beam 5 % and more;
  *  - the kick's Fx term, ((ds (1 + X/rho0)) 0)/rho_actual, is a signed zero;
  *  - dz_lost is summed only for a lost particle, from the substeps done.
  * Loss conditions, their order and the state left at a loss are the
@@ -1851,10 +1853,9 @@ __device__ __forceinline__ bool op_bend(const trk_op *__restrict__ op, Part &p, 
 /* op_mult restricted to OPK_MULT1 (one normal multipole, 4th-order integrator
  * with drifts, no misalignment, steering, radiation or fringe), with the same
  * roundings:
- *  - the first conversion to slopes after a kick is used for its loss test
- *    only, the one after the (1 + delta) round trip gives the slopes; the two
- *    share the root and its reciprocal while their radicands are equal, which
- *    the ulp the trip can move a momentum by hardly ever changes;
+ *  - of the first conversion to slopes after a kick only the loss test is left,
+ *    the sign of its radicand; the one after the (1 + delta) round trip gives
+ *    the slopes;
  *  - quotients by 1 + delta and by the roots through their correctly rounded
  *    reciprocals (trkcr_div_rcp);
  *  - the conversion after the last drift repeats the last kick's;
@@ -2397,7 +2398,7 @@ template <bool WIDE> __device__ __forceinline__ unsigned entry_z(double ss) {
  * Such a warp takes the wide body at once.  Where both accept a particle they
  * do the same operations, so its track does not depend on its neighbours. */
 #define TRK_STEEP_MULT 0x3f86a09eu /* 2^-6.5 in each plane: z = 2^-12 */
-#define TRK_STEEP_BEND 0x3f747ae1u /* 0.005: the bend's own swing adds up to 0.0085 (trk_compile) */
+#define TRK_STEEP_BEND 0x3f747ae1u /* 0.005: the bend's own swing adds up to 0.010 (trk_compile) */
 __device__ __forceinline__ bool warp_steep(const Part &p, unsigned limit) {
   return __any_sync(__activemask(), max(hi_abs(p.xp), hi_abs(p.yp)) >= limit);
 }
@@ -2648,13 +2649,21 @@ __device__ __forceinline__ bool cfbend_merged(const double *__restrict__ d, cons
 /* The other bodies out of line, for the particles the narrow ones leave,
  * passed and returned by value (a reference would pin the caller's
  * coordinates in local memory): the wide merged body, and the checked one for
- * what is near a loss.  All elements inside an aperture take the checked one:
- * particles near the dynamic aperture move chaotically, and any other order
- * of rounding changes their tracks by up to 1e-4 of the beam after 32 turns,
- * so aperture studies keep the unmerged arithmetic.  What they do not need is
- * the test in every slice, with its divisions: the body runs without it and
- * the box around the slice boundaries is tested in products; only a particle
- * whose box is not clear of the aperture is taken through the tests. */
+ * what is near a loss.  All elements inside an aperture take the checked one.
+ * That is not for accuracy: of particles on a dynamic-aperture grid, 32 turns
+ * on, the merged tracks are the nearer to an 80-bit restatement (4.4e-10 of the
+ * beam against 7.7e-10, geometric means over 12 error seeds).  But such
+ * particles move chaotically, any other order of rounding changes their tracks
+ * by up to 1e-4 of the beam in that time, and aperture studies were to keep the
+ * tracks they had.  A MAXAMP stands for such a study, so a ring with nothing
+ * but a wide chamber takes these bodies too (radiating elements do not).  What
+ * they do not need is the test in every slice, with its divisions: the body
+ * runs without it and the box around the slice boundaries is tested in
+ * products; only a particle whose box is not clear of the aperture is taken
+ * through the tests.  (A beam that loses three quarters of its particles in 40
+ * elements pays for both: 1.13 times the tests alone with a rectangle, 1.01 with
+ * an ellipse.  One body with cheap tests is 1.0 and 0.8 there, but 4 % slower
+ * for beams well inside.) */
 template <int ORDER>
 __device__ __forceinline__ bool mult1_wide(const trk_op *__restrict__ op, Part &p) {
   return mult1_merged<ORDER, true>(op->d, __ldg(&op->i[0]), p);
@@ -3837,13 +3846,13 @@ __global__ void matrix_kernel(TrackArgs a, const double *__restrict__ m, int ord
  * atomic per warp and element.  delta has no adjoint: nothing on this path
  * changes it.
  *
- * Bound by FP64 issue and the length of a substep's chain (60 % of the FP64
- * pipe with every SM full): about 43 operations per substep of a dipole and
+ * Bound by FP64 issue and the length of a substep's chain (54 % of the FP64
+ * pipe at 1e5 particles): about 43 operations per substep of a dipole and
  * 25 more for the K1 and K2 sensitivities of its kick.  Measured on the FODO
- * ring with sextupoles, 1e5 particles, per turn, forward pass included: 4.8
+ * ring with sextupoles, 1e5 particles, per turn, forward pass included: 4.9
  * ms; recording every element's entry state and every substep's in local
- * memory took 14.5 ms and 9 GB of memory traffic.  (128, 4) with 122
- * registers: (128, 6) with 80 is 1 % slower at 1e5 particles and more, 7 %
+ * memory took 14.5 ms and 9 GB of memory traffic.  (128, 4) with 108
+ * registers: (128, 6) with 80 was 1 % slower at 1e5 particles and more, 7 %
  * below a block per SM. */
 
 /* 1/sqrt(1 - z) and sqrt(1 - z) = (1 - z)/sqrt(1 - z) for any z < 1 */

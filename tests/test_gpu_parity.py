@@ -167,11 +167,11 @@ def test_fodo_ring_fast_one_turn(tracker):
     assert r["max_err"] < 2e-8, r
 
 
-@pytest.mark.parametrize("variant", range(7))
+@pytest.mark.parametrize("variant", (0, 1, 2, 3, 4, 7, 8))
 def test_kernel_variants_fast_losses(tracker, variant):
-    """Every launch shape of the fast tracking kernel (one and two particles
-    per thread) against the oracle on a lossy ring: same survivors, same loss
-    pass and element, coordinates within the fast build's bound."""
+    """Every launch shape of the fast tracking kernel against the oracle on a
+    lossy ring: same survivors, same loss pass and element, coordinates within
+    the fast build's bound."""
     lat = Lattice()
     lat.add("MAXAMP", "AP", X_MAX=0.004, Y_MAX=0.003, ELLIPTICAL=1)
     lat.extend(configs.c1_lattice(cells=4))
@@ -187,6 +187,25 @@ def test_kernel_variants_fast_losses(tracker, variant):
     gi = np.argsort(g[:, 6])
     assert np.array_equal(lp[gi][lost], o[lost, 7].astype(np.int64))
     assert np.array_equal(le[gi][lost], o[lost, 8].astype(np.int32))
+
+
+@pytest.mark.parametrize("fast", [True, False])
+@pytest.mark.parametrize("ring", ["fodo_sext", "mba"])
+@pytest.mark.parametrize("variant", (0, 1, 2, 3, 4, 7, 8))
+def test_kernel_variants_without_apertures(tracker, variant, ring, fast):
+    """Every launch shape, large beams' defaults (4, 7) among them, through the
+    merged bodies of both lean flavours (the achromat ring holds
+    combined-function bends) and through the parity build."""
+    if ring == "mba":
+        lat, beam = configs.c5_lattice(cells=1, with_rf=False, with_wake=False), configs.c5_beam(1001, seed=9)
+    else:
+        lat, beam = configs.c2_lattice(cells=4, with_rf=False, with_wake=False), configs.gaussian_beam(3001, seed=9)
+    nl, g, lp, le, _ = gpu_run(tracker, lat, beam, 2, PC, fast=fast, variant=variant)
+    with pyoracle.modes(exact_sums=True, cr_math=True):
+        rows, nlo, _ = oracle_run(lat, beam, 2, PC)
+    r = compare(g, rows, nl, nlo)
+    assert nlo == beam.shape[0] and r["same_survivors"]
+    assert r["max_err"] < 2e-8 if fast else r["bit_exact"], r
 
 
 def test_losses_rect_aperture_exact(tracker):
