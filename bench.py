@@ -24,10 +24,11 @@ value : particle-turns/s with the beam resident on the device; each step is
         (a 512 MiB write) between timed steps and outside their events.
 e2e   : the same metric through the C ABI with host buffers: each step loads
         the beam from pinned host memory, tracks one turn and stores it back.
-roofline: FP64 bound; achieved = algorithmic FP64 flops per particle-turn
-        (counted on the reference formulation, oracle/flops.json) times
+roofline: FP64 bound; achieved = FP64 flops per particle-turn times
         particle-turns/s, against the FP64 peak measured in this run by a
-        dependent-FMA kernel (MEASURED_PEAKS.json has no FP64 figure).
+        dependent-FMA kernel (MEASURED_PEAKS.json has no FP64 figure).  The
+        parity build's flops are counted on the reference formulation
+        (oracle/flops.json), the fast build's on its own, which needs fewer.
 --impl reference: elegant's own tracking code compiled from the reference
         sources (oracle/_ref/libref.so; the oracle restatement where that
         was not built) on all host cores, process-parallel by particle
@@ -55,12 +56,12 @@ ROOT = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, ROOT)
 
 N_PARTICLES = 1_000_000
-# DRAM bytes per particle of one tracking-kernel launch: 10.63 MB read + 1.8 KB
-# written at 2e5 particles (ncu; the coordinate writes stay in L2 and are
-# written back during later kernels)
-TRACK_DRAM_BYTES_PER_PARTICLE = 10.628e6 / 2e5
-# the same for the MBA ring: 110.67 MB read + 120.53 MB written at 2e6 particles (ncu)
-TRACK_DRAM_BYTES_PER_PARTICLE_C5 = (110.67e6 + 120.53e6) / 2e6
+# DRAM bytes per particle of one tracking-kernel launch: fast build 10.7 MB read
+# + 11 KB written at 2e5 particles, parity build 6.2 MB + 0.86 MB at 1e5 (ncu; the
+# coordinate writes stay in L2 and are written back during later kernels)
+TRACK_DRAM_BYTES_PER_PARTICLE = {True: 10.711e6 / 2e5, False: 7.06e6 / 1e5}
+# the same for the MBA ring, fast build: 108.8 MB read + 53.7 MB written at 2e6 particles (ncu)
+TRACK_DRAM_BYTES_PER_PARTICLE_C5 = (108.8e6 + 53.7e6) / 2e6
 
 WORKLOADS = {
     "c1": {"workload": "ring_fodo40_1e6", "particles": 1_000_000,
@@ -811,30 +812,52 @@ def _e2e(trk, lat, fast, beam, steps, world):
             "h2d_bytes_per_step": int(n * 7 * 8), "d2h_bytes_per_step": int(n * 7 * 8)}
 
 
-def _roofline(m, workload, world, peak, flops):
-    """FP64 roofline of the fused tracking kernel: algorithmic flops of the
-    elements it runs (reference formulation, oracle/flops.json) per launch
-    over its CUDA-event launch time."""
+def _merged_flops(lat):
+    """FP64 flops of one particle and turn in the fast build's merged bodies
+    (a multiply-add is two): per kick and the drift after it 25 in a
+    multipole, 35 in a dipole, 60 in one with a gradient, three of them to a
+    slice and one drift more; 11 in any other element."""
+    f = 0
+    for kind, _, p, _ in lat.elements:
+        if kind in ("KQUAD", "KSEXT", "KOCT"):
+            f += 25 * (3 * p["N_KICKS"] // 4 + 1)
+        elif kind == "CSBEND":
+            f += (60 if p.get("K1") else 35) * (3 * p["N_KICKS"] + 1)
+        else:
+            f += 11
+    return f
+
+
+def _roofline(m, workload, world, peak, flops, fast):
+    """FP64 roofline of the fused tracking kernel: flops of the elements it
+    runs (parity build: reference formulation, oracle/flops.json; fast build:
+    its own) per launch over its CUDA-event launch time."""
     if not flops or not m["track_launches"]:
         return None
+    if fast:
+        fpt = _merged_flops(workload_lattice("c2" if workload == "rad" else workload))
+    else:
+        fpt = flops["flops_per_particle_turn"]["c2" if workload == "rad" else workload]
+        # the wakes' per-particle work runs in the wake kernels
+        fpt -= {"c1": 0, "c2": 1, "rad": 1, "c5": 2}[workload] * flops["per_particle"]["WAKE"]["total"]
     # the radiating ring is counted as the plain one (the radiation's own flops are not counted)
-    fpt = flops["flops_per_particle_turn"]["c2" if workload == "rad" else workload]
-    # the wakes' per-particle work runs in the wake kernels
-    fpt -= {"c1": 0, "c2": 1, "rad": 1, "c5": 2}[workload] * flops["per_particle"]["WAKE"]["total"]
     per_launch_flops = fpt * (m["effort"] / world) / m["track_launches"]
     avg_launch_s = m["track_ms"] / m["track_launches"] / 1e3
     achieved = per_launch_flops / avg_launch_s / 1e12
-    traffic = {"c2": TRACK_DRAM_BYTES_PER_PARTICLE, "c5": TRACK_DRAM_BYTES_PER_PARTICLE_C5}.get(workload)
+    traffic = {"c2": TRACK_DRAM_BYTES_PER_PARTICLE[fast], "c5": TRACK_DRAM_BYTES_PER_PARTICLE_C5 if fast else None}.get(workload)
     return {"bound": "fp64", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
             "frac": achieved / peak if peak else None,
             "traffic": traffic * (m["effort"] / world) / m["track_launches"] if traffic else None,
-            "flops_per_particle_turn": fpt, "kernel": "track_kernel", "launches": m["track_launches"],
+            "flops_per_particle_turn": fpt,
+            "flops_counted_on": "the merged bodies" if fast else "the reference formulation",
+            "kernel": "track_kernel", "launches": m["track_launches"],
             "avg_launch_ms": avg_launch_s * 1e3,
             "peak_source": "FP64 FMA peak measured in this run (independent dependent-FMA chains); "
                            "MEASURED_PEAKS.json has no FP64 figure",
             "traffic_source": (None if not traffic else
-                               "ncu dram__bytes_read.sum + dram__bytes_write.sum of one fast-build launch at "
-                               + ("2e5" if workload == "c2" else "2e6") + " particles, scaled by particles")}
+                               "ncu dram__bytes_read.sum + dram__bytes_write.sum of one launch at "
+                               + (("2e5" if fast else "1e5") if workload == "c2" else "2e6")
+                               + " particles, scaled by particles")}
 
 
 LONG_FIXTURES = os.path.join(ROOT, "tests", "golden", "long_tracks.npz")
@@ -935,7 +958,7 @@ def run_gpu(args, rank, world, local):
             "higher_is_better": True, "scaling": "weak", "vs_baseline": None, "dtype": "f64",
             "data": "synthetic (seeded Gaussian beam, seeded resonator wake)",
             "config": workload_config(n, args.workload), "build": head, "wall_s": m["wall"], "e2e": m["e2e"],
-            "gpu_launches": m["launches"], "roofline": _roofline(m, args.workload, world, peak, flops),
+            "gpu_launches": m["launches"], "roofline": _roofline(m, args.workload, world, peak, flops, head == "fast"),
             "cpu_baseline": cpu, "clocks": m["clocks"]}
     if acc and acc.get(head):
         line["accuracy"] = acc[head]
@@ -946,7 +969,7 @@ def run_gpu(args, rank, world, local):
         mb = res[b]
         line[f"{b}_build"] = {"value": mb["value"], "ms_per_step": mb["dev_s"] * 1e3 / args.steps,
                               "e2e": mb["e2e"], "gpu_launches": mb["launches"],
-                              "roofline": _roofline(mb, args.workload, world, peak, flops),
+                              "roofline": _roofline(mb, args.workload, world, peak, flops, b == "fast"),
                               "accuracy": acc.get(b) if acc else None, "clocks": mb["clocks"]}
     print(json.dumps(line), flush=True)
     return 0
