@@ -1996,9 +1996,10 @@ static int adjoint_run(trk_context *ctx, const trk_lattice *const *lattices, int
         return trk_set_error(TRK_ERR_UNSUPPORTED, "CSBEND with more than 32 slices in a gradient run");
       break;
     default:
-      return trk_set_error(TRK_ERR_UNSUPPORTED, "variant %d, element %d: gradients cover DRIF, EDRIFT, KQUAD/KSEXT/"
-                           "KOCT (single order, no tilt or misalignment) and CSBEND (pure dipole or K1/K2 "
-                           "expansion, no misalignment or edge kick)", k / nops, op.elem);
+      return trk_set_error(TRK_ERR_UNSUPPORTED, "%selement %d: gradients cover DRIF, EDRIFT, KQUAD/KSEXT/KOCT "
+                           "(single order, no tilt or misalignment) and CSBEND (pure dipole or K1/K2 "
+                           "expansion, no misalignment or edge kick)",
+                           ensemble ? ("variant " + std::to_string(k / nops) + ", ").c_str() : "", op.elem);
     }
   }
   for (int k = 0; k < nops; k++) {

@@ -2340,8 +2340,8 @@ __device__ __forceinline__ bool op_cfbend_fast(const trk_op *__restrict__ op, Pa
  * Slopes above the polynomials' range take the same bodies with roots (WIDE).
  * Bound by FP64 issue and by the length of the substep's chain (13 of its 17
  * operations).  Measured against the checked bodies alone, ms per turn: FODO
- * ring with RF and wake, 1e6 particles, 11.4 -> 7.5; achromat ring, 2e6, 250
- * -> 149; FODO ring, 1e4 particles, 0.67 -> 0.36. */
+ * ring with RF and wake, 1e6 particles, 11.4 -> 7.6; achromat ring, 2e6, 250
+ * -> 150; FODO ring, 1e4 particles, 0.67 -> 0.36. */
 
 /* Coefficients: the power series, its first omitted term economized over
  * [0, b], b = 2^-12 (z^4 replaced by z^4 - b^4 T4*(z/b)/128 without the
@@ -2396,7 +2396,9 @@ template <bool WIDE> __device__ __forceinline__ unsigned entry_z(double ss) {
 /* whether a lane of the warp enters with a slope at which the narrow body may
  * end up above its bound (high word of the slope below which it does not).
  * Such a warp takes the wide body at once.  Where both accept a particle they
- * do the same operations, so its track does not depend on its neighbours. */
+ * do the same operations, so its track does not depend on its neighbours, nor
+ * on which lanes happen to vote together.  The vote costs 1 % of the rings'
+ * times (FODO ring, 1e4 particles x 100 turns: 36.0 -> 36.4 ms). */
 #define TRK_STEEP_MULT 0x3f86a09eu /* 2^-6.5 in each plane: z = 2^-12 */
 #define TRK_STEEP_BEND 0x3f747ae1u /* 0.005: the bend's own swing adds up to 0.010 (trk_compile) */
 __device__ __forceinline__ bool warp_steep(const Part &p, unsigned limit) {
